@@ -15,9 +15,8 @@
 //              and shared memory, arg-max written per ray
 //   training   softmax cross-entropy against the cluster of the ray's first
 //              hit (records from earlier batches), plain minibatch SGD with
-//              momentum; every GEMM of the forward and backward pass is the
-//              tcgen05 GEMM of pbg_mlp.cu, with small CUDA-core kernels for
-//              bias, ReLU, softmax, transposes and the update.
+//              momentum: one kernel for the forward and backward pass and one
+//              for the update per step (pbg_train.cu).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -27,10 +26,6 @@
 #include "pbg_tc.cuh"
 
 namespace pbg {
-
-int tc_gemm(const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int accumulate,
-            int* status, cudaStream_t st, float* work);
-size_t tc_gemm_work_floats(int M, int N, int K);
 
 // ------------------------------------------------------------ features
 
@@ -68,163 +63,6 @@ __device__ __forceinline__ void for_each_feature(float4 o, float4 d, const float
     for (int k = 9 + 96; k < kFeat; ++k) emit(0.f);
 }
 
-__device__ __forceinline__ void ray_features(float4 o, float4 d, const float* lo, const float* inv_ext,
-                                             float* f /* kFeat */) {
-    int k = 0;
-    for_each_feature(o, d, lo, inv_ext, [&](float v) { f[k++] = v; });
-}
-
-// X [n_pad x 112] bf16 rows; rows >= n are zero.
-__global__ void features_kernel(const float4* __restrict__ ro, const float4* __restrict__ rd,
-                                const int32_t* __restrict__ idx, int64_t n, int64_t n_pad,
-                                LearnBox box, uint16_t* __restrict__ X) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pad) return;
-    float f[kFeat];
-    if (i < n) {
-        const int64_t r = idx ? (int64_t)idx[i] : i;
-        ray_features(ro[r], rd[r], box.lo, box.inv_ext, f);
-    } else {
-        for (int k = 0; k < kFeat; ++k) f[k] = 0.f;
-    }
-    uint16_t* row = X + i * kFeat;
-#pragma unroll
-    for (int k = 0; k < kFeat; ++k) row[k] = f2bf(f[k]);
-}
-
-// ------------------------------------------------------- training step
-
-// H = relu(Z + b) as bf16 (row-major [rows x cols]); Z fp32 in place kept.
-__global__ void bias_relu_kernel(float* __restrict__ Z, const float* __restrict__ b, int64_t rows,
-                                 int cols, int relu, uint16_t* __restrict__ H) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    const int c = (int)(i % cols);
-    float v = Z[i] + b[c];
-    if (relu) v = fmaxf(v, 0.f);
-    Z[i] = v;
-    if (H) H[i] = f2bf(v);
-}
-
-// dZ = (softmax(Z) - onehot(label)) / B for valid rows; loss and accuracy
-// accumulated in acc[0..1].  One warp per row of 256 logits.
-__global__ void softmax_grad_kernel(const float* __restrict__ Z, const int32_t* __restrict__ label,
-                                    int64_t rows, int64_t valid_rows, float scale,
-                                    float* __restrict__ dZ, uint16_t* __restrict__ dZb,
-                                    float* __restrict__ acc) {
-    const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (r >= rows) return;
-    const float* z = Z + r * kClusters;
-    float v[8];
-    float mx = -INFINITY;
-    int am = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        v[k] = z[lane + 32 * k];
-        if (v[k] > mx) {
-            mx = v[k];
-            am = lane + 32 * k;
-        }
-    }
-    for (int off = 16; off; off >>= 1) {
-        const float om = __shfl_xor_sync(0xffffffffu, mx, off);
-        const int oa = __shfl_xor_sync(0xffffffffu, am, off);
-        if (om > mx || (om == mx && oa < am)) {
-            mx = om;
-            am = oa;
-        }
-    }
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        v[k] = __expf(v[k] - mx);
-        s += v[k];
-    }
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    const bool ok = r < valid_rows;
-    const int y = ok ? label[r] : -1;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int c = lane + 32 * k;
-        float g = ok ? (v[k] / s - (c == y ? 1.f : 0.f)) * scale : 0.f;
-        dZ[r * kClusters + c] = g;
-        dZb[r * kClusters + c] = f2bf(g);
-        if (ok && c == y && lane == (y & 31)) {
-            atomicAdd(&acc[0], -__logf(fmaxf(v[k] / s, 1e-30f)));
-            if (am == y) atomicAdd(&acc[1], 1.f);
-        }
-    }
-}
-
-// T[cols_pad x rows] = M[rows x cols]^T (bf16), rows beyond `cols` zero.
-__global__ void transpose_bf16_kernel(const uint16_t* __restrict__ M, int64_t rows, int cols,
-                                      int cols_pad, uint16_t* __restrict__ T) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols_pad) return;
-    const int c = (int)(i / rows);
-    const int64_t r = i % rows;
-    T[i] = c < cols ? M[r * cols + c] : (uint16_t)0;
-}
-
-// dH (fp32) -> dZ = dH * (Zact > 0), kept in place (for the bias sums) and
-// as bf16 (for the next GEMMs)
-__global__ void relu_grad_kernel(float* __restrict__ dH, const float* __restrict__ Zact, int64_t n,
-                                 uint16_t* __restrict__ dZ) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = Zact[i] > 0.f ? dH[i] : 0.f;
-    dH[i] = v;
-    dZ[i] = f2bf(v);
-}
-
-// column sums of dZ [rows x cols] into db
-__global__ void colsum_kernel(const float* __restrict__ dZ, int64_t rows, int cols, float* __restrict__ db) {
-    const int c = blockIdx.x;
-    float s = 0.f;
-    for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) s += dZ[r * cols + c];
-    for (int off = 16; off; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    __shared__ float ws[32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += ws[w];
-        db[c] = t;
-    }
-}
-
-// SGD with momentum on FP32 master weights; refreshes the BF16 copies in
-// both orientations (out x in for the forward GEMMs, in x out for dH).
-__global__ void sgd_kernel(float* __restrict__ W, float* __restrict__ V, const float* __restrict__ G,
-                           int out, int in, int in_pad, float lr, float mom,
-                           uint16_t* __restrict__ Wb, uint16_t* __restrict__ WbT, int out_padT) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= out * in_pad) return;
-    const int o = i / in_pad, k = i % in_pad;
-    if (k >= in) {
-        Wb[i] = 0;
-        return;
-    }
-    const float g = G[(size_t)o * in_pad + k];
-    float v = mom * V[i] + g;
-    V[i] = v;
-    const float w = W[i] - lr * v;
-    W[i] = w;
-    const uint16_t h = f2bf(w);
-    Wb[i] = h;
-    if (WbT) WbT[(size_t)k * out_padT + o] = h;
-}
-
-__global__ void sgd_bias_kernel(float* __restrict__ b, float* __restrict__ v, const float* __restrict__ g,
-                                int n, float lr, float mom) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float vv = mom * v[i] + g[i];
-    v[i] = vv;
-    b[i] -= lr * vv;
-}
-
 // ------------------------------------------------------------ inference
 
 constexpr int kInferThreads = 128;
@@ -248,12 +86,7 @@ __device__ __forceinline__ void stage_rows(uint8_t* dst, const uint16_t* src, in
 
 // Eight values as bf16 into a row's group of a core-matrix tile.
 __device__ __forceinline__ void store_group(uint8_t* dst, int r, int g, int cols, const float* v) {
-    uint4 w;
-    w.x = (uint32_t)f2bf(v[0]) | ((uint32_t)f2bf(v[1]) << 16);
-    w.y = (uint32_t)f2bf(v[2]) | ((uint32_t)f2bf(v[3]) << 16);
-    w.z = (uint32_t)f2bf(v[4]) | ((uint32_t)f2bf(v[5]) << 16);
-    w.w = (uint32_t)f2bf(v[6]) | ((uint32_t)f2bf(v[7]) << 16);
-    *(uint4*)(dst + core_offset(r, g, cols)) = w;
+    *(uint4*)(dst + core_offset(r, g, cols)) = pack8(v);
 }
 
 // A ray's features straight into its row of the X tile, eight at a time.
@@ -407,9 +240,7 @@ __global__ void __launch_bounds__(kInferThreads)
 
 // ---------------------------------------------------------- host logic
 
-static int upload_params(Learner* L, const std::vector<float>& w1, const std::vector<float>& b1,
-                         const std::vector<float>& w2, const std::vector<float>& b2,
-                         const std::vector<float>& w3, const std::vector<float>& b3, cudaStream_t st);
+static int upload_params(Learner* L, const float* params, cudaStream_t st);
 
 // Child references of the BVH cut into up to kClusters subtrees: starting
 // from the root's two children, the largest inner subtree is split until
@@ -472,16 +303,13 @@ static void build_clusters(const std::vector<BvhNode>& nodes, int64_t nrec, std:
 
 void learn_free(Learner* L) {
     if (!L) return;
-    DeviceBuffer* all[] = {&L->cluster_ref, &L->record_cluster, &L->W1, &L->W2, &L->W3, &L->V1, &L->V2,
-                           &L->V3, &L->b1, &L->b2, &L->b3, &L->vb1, &L->vb2, &L->vb3, &L->W1b, &L->W2b,
-                           &L->W3b, &L->W2Tb, &L->W3Tb, &L->recX, &L->recY, &L->X, &L->XT, &L->Z1,
-                           &L->Z2, &L->Z3, &L->H1, &L->H2, &L->H1T, &L->H2T, &L->dZ3, &L->dZ3b,
-                           &L->dZ3T, &L->dH2, &L->dZ2b, &L->dZ2T, &L->dH1, &L->dZ1b, &L->dZ1T, &L->G1,
-                           &L->G2, &L->G3, &L->gb1, &L->gb2, &L->gb3, &L->acc, &L->feat, &L->pred,
-                           &L->gemm_work, &L->occ_prim};
+    DeviceBuffer* all[] = {&L->cluster_ref, &L->record_cluster, &L->P, &L->V, &L->Wb, &L->G, &L->part, &L->acc,
+                           &L->recX, &L->recY, &L->X, &L->feat, &L->pred, &L->occ_prim};
     for (DeviceBuffer* b : all) release(*b);
     for (cudaEvent_t e : L->infer_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : L->infer_pool) cudaEventDestroy(e);
+    for (cudaEvent_t e : L->train_ev)
+        if (e) cudaEventDestroy(e);
     delete L;
 }
 
@@ -547,11 +375,11 @@ int learn_init(pbg_scene* s, const pbg_learn_params* p) {
         if (p->lr > 0.f) L->lr = p->lr;
         if (p->margin != 0.f) L->margin = p->margin;
         if (p->momentum > 0.f) L->momentum = p->momentum;
-        if (p->records > 0 && !L->W1.ptr) L->capacity = p->records;  // the ring is sized once
+        if (p->records > 0 && !L->P.ptr) L->capacity = p->records;  // the ring is sized once
         if (p->seed) L->seed = p->seed;
     }
     if (p && p->queries > 0) L->queries = p->queries & 3;
-    if (L->W1.ptr) {  // initialised before: keep the weights and records
+    if (L->P.ptr) {  // initialised before: keep the weights and records
         L->enabled = true;
         return PBG_OK;
     }
@@ -571,13 +399,12 @@ int learn_init(pbg_scene* s, const pbg_learn_params* p) {
         return (double)((z * 2685821657736338717ull) >> 11) * (1.0 / 9007199254740992.0);
     };
     auto normal = [&]() { return std::sqrt(-2.0 * std::log(u01() + 1e-300)) * std::cos(6.283185307179586 * u01()); };
-    std::vector<float> w1((size_t)kHidden * kFeat, 0.f), w2((size_t)kHidden * kHidden), w3((size_t)kClusters * kHidden);
-    std::vector<float> b1(kHidden, 0.f), b2(kHidden, 0.f), b3(kClusters, 0.f);
+    std::vector<float> w(kParams, 0.f);  // biases and padding columns zero
     for (int o = 0; o < kHidden; ++o)
-        for (int k = 0; k < 105; ++k) w1[(size_t)o * kFeat + k] = (float)(normal() * std::sqrt(2.0 / 105));
-    for (auto& w : w2) w = (float)(normal() * std::sqrt(2.0 / kHidden));
-    for (auto& w : w3) w = (float)(normal() * std::sqrt(1.0 / kHidden));
-    if ((rc = upload_params(L, w1, b1, w2, b2, w3, b3, st))) return rc;
+        for (int k = 0; k < 105; ++k) w[kOffW1 + (size_t)o * kFeat + k] = (float)(normal() * std::sqrt(2.0 / 105));
+    for (int k = 0; k < kHidden * kHidden; ++k) w[kOffW2 + (size_t)k] = (float)(normal() * std::sqrt(2.0 / kHidden));
+    for (int k = 0; k < kClusters * kHidden; ++k) w[kOffW3 + (size_t)k] = (float)(normal() * std::sqrt(1.0 / kHidden));
+    if ((rc = upload_params(L, w.data(), st))) return rc;
     L->enabled = true;
     L->count = L->head = 0;
     if ((rc = ensure(L->acc, 64))) return rc;
@@ -586,43 +413,19 @@ int learn_init(pbg_scene* s, const pbg_learn_params* p) {
     return PBG_OK;
 }
 
-// Uploads FP32 parameters, zeroes momentum, refreshes the BF16 copies.
-__global__ void to_bf16_kernel(const float* __restrict__ W, int out, int in, uint16_t* __restrict__ Wb,
-                               uint16_t* __restrict__ WbT) {
+__global__ void to_bf16_kernel(const float* __restrict__ P, uint16_t* __restrict__ Wb) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= out * in) return;
-    const int o = i / in, k = i % in;
-    const uint16_t h = f2bf(W[i]);
-    Wb[i] = h;
-    if (WbT) WbT[(size_t)k * out + o] = h;
+    if (i < kParams) Wb[i] = f2bf(P[i]);
 }
 
-static int upload_params(Learner* L, const std::vector<float>& w1, const std::vector<float>& b1,
-                         const std::vector<float>& w2, const std::vector<float>& b2,
-                         const std::vector<float>& w3, const std::vector<float>& b3, cudaStream_t st) {
+// Uploads FP32 parameters, zeroes momentum, refreshes the BF16 copies.
+static int upload_params(Learner* L, const float* params, cudaStream_t st) {
     int rc;
-    const size_t n1 = (size_t)kHidden * kFeat, n2 = (size_t)kHidden * kHidden, n3 = (size_t)kClusters * kHidden;
-    if ((rc = ensure(L->W1, n1 * 4)) || (rc = ensure(L->W2, n2 * 4)) || (rc = ensure(L->W3, n3 * 4)) ||
-        (rc = ensure(L->V1, n1 * 4)) || (rc = ensure(L->V2, n2 * 4)) || (rc = ensure(L->V3, n3 * 4)) ||
-        (rc = ensure(L->b1, kHidden * 4)) || (rc = ensure(L->b2, kHidden * 4)) || (rc = ensure(L->b3, kClusters * 4)) ||
-        (rc = ensure(L->vb1, kHidden * 4)) || (rc = ensure(L->vb2, kHidden * 4)) || (rc = ensure(L->vb3, kClusters * 4)) ||
-        (rc = ensure(L->W1b, n1 * 2)) || (rc = ensure(L->W2b, n2 * 2)) || (rc = ensure(L->W3b, n3 * 2)) ||
-        (rc = ensure(L->W2Tb, n2 * 2)) || (rc = ensure(L->W3Tb, n3 * 2)))
+    if ((rc = ensure(L->P, kParams * 4)) || (rc = ensure(L->V, kParams * 4)) || (rc = ensure(L->Wb, kParams * 2)))
         return rc;
-    PBG_CUDA(cudaMemcpyAsync(L->W1.ptr, w1.data(), n1 * 4, cudaMemcpyHostToDevice, st));
-    PBG_CUDA(cudaMemcpyAsync(L->W2.ptr, w2.data(), n2 * 4, cudaMemcpyHostToDevice, st));
-    PBG_CUDA(cudaMemcpyAsync(L->W3.ptr, w3.data(), n3 * 4, cudaMemcpyHostToDevice, st));
-    PBG_CUDA(cudaMemcpyAsync(L->b1.ptr, b1.data(), kHidden * 4, cudaMemcpyHostToDevice, st));
-    PBG_CUDA(cudaMemcpyAsync(L->b2.ptr, b2.data(), kHidden * 4, cudaMemcpyHostToDevice, st));
-    PBG_CUDA(cudaMemcpyAsync(L->b3.ptr, b3.data(), kClusters * 4, cudaMemcpyHostToDevice, st));
-    DeviceBuffer* zero[] = {&L->V1, &L->V2, &L->V3, &L->vb1, &L->vb2, &L->vb3};
-    for (DeviceBuffer* b : zero) PBG_CUDA(cudaMemsetAsync(b->ptr, 0, b->bytes, st));
-    to_bf16_kernel<<<(unsigned)((n1 + 255) / 256), 256, 0, st>>>((const float*)L->W1.ptr, kHidden, kFeat,
-                                                                  (uint16_t*)L->W1b.ptr, nullptr);
-    to_bf16_kernel<<<(unsigned)((n2 + 255) / 256), 256, 0, st>>>((const float*)L->W2.ptr, kHidden, kHidden,
-                                                                  (uint16_t*)L->W2b.ptr, (uint16_t*)L->W2Tb.ptr);
-    to_bf16_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>((const float*)L->W3.ptr, kClusters, kHidden,
-                                                                  (uint16_t*)L->W3b.ptr, (uint16_t*)L->W3Tb.ptr);
+    PBG_CUDA(cudaMemcpyAsync(L->P.ptr, params, kParams * 4, cudaMemcpyHostToDevice, st));
+    PBG_CUDA(cudaMemsetAsync(L->V.ptr, 0, kParams * 4, st));
+    to_bf16_kernel<<<(kParams + 255) / 256, 256, 0, st>>>((const float*)L->P.ptr, (uint16_t*)L->Wb.ptr);
     PBG_CUDA(cudaGetLastError());
     PBG_CUDA(cudaStreamSynchronize(st));
     return PBG_OK;
@@ -675,9 +478,9 @@ int learn_predict(pbg_scene* s, const float4* o, const float4* d, int64_t n, con
     PBG_CUDA(cudaEventRecord(ev[0], st));
     prof_begin(s, st);
     mlp_infer_kernel<<<grid, kInferThreads, kInferSmem, st>>>(
-        o, d, n, L->box, (const uint16_t*)L->W1b.ptr, (const uint16_t*)L->W2b.ptr, (const uint16_t*)L->W3b.ptr,
-        (const float*)L->b1.ptr, (const float*)L->b2.ptr, (const float*)L->b3.ptr, L->margin,
-        (uint16_t*)L->pred.ptr, (int*)s->err.ptr);
+        o, d, n, L->box, (const uint16_t*)L->Wb.ptr + kOffW1, (const uint16_t*)L->Wb.ptr + kOffW2,
+        (const uint16_t*)L->Wb.ptr + kOffW3, (const float*)L->P.ptr + kOffB1, (const float*)L->P.ptr + kOffB2,
+        (const float*)L->P.ptr + kOffB3, L->margin, (uint16_t*)L->pred.ptr, (int*)s->err.ptr);
     prof_end(s, st, kStageOther, 1);
     PBG_CUDA(cudaGetLastError());
     PBG_CUDA(cudaEventRecord(ev[1], st));
@@ -705,10 +508,16 @@ __global__ void collect_kernel(const float4* __restrict__ ro, const float4* __re
     const unsigned int k = atomicAdd(taken, 1u);
     if ((int64_t)k >= take) return;
     const int64_t slot = (int64_t)((*total + k) % (unsigned long long)cap);
-    float f[kFeat];
-    ray_features(ro[i], rd[i], box.lo, box.inv_ext, f);
-    uint16_t* row = recX + slot * kFeat;
-    for (int j = 0; j < kFeat; ++j) row[j] = f2bf(f[j]);
+    uint4* row = (uint4*)(recX + slot * kFeat);  // 224-byte rows: eight features per store
+    float buf[8];
+    int m = 0, g = 0;
+    for_each_feature(ro[i], rd[i], box.lo, box.inv_ext, [&](float v) {
+        buf[m++] = v;
+        if (m == 8) {
+            row[g++] = pack8(buf);
+            m = 0;
+        }
+    });
     recY[slot] = c;
 }
 
@@ -745,122 +554,15 @@ int learn_collect(pbg_scene* s, const float4* o, const float4* d, const int32_t*
 }
 
 // Records collected so far (a synchronising read of the device total).
-static int records_available(Learner* L, cudaStream_t st) {
+static int records_available(pbg_scene* s, Learner* L, cudaStream_t st) {
     unsigned long long total = 0;
     if (L->acc.ptr) {
-        PBG_CUDA(cudaMemcpyAsync(&total, (uint8_t*)L->acc.ptr + 40, 8, cudaMemcpyDeviceToHost, st));
-        PBG_CUDA(cudaStreamSynchronize(st));
+        int w[2] = {0, 0};
+        const int rc = read_device_words(s, (const int*)L->acc.ptr + 10, 2, w, st);
+        if (rc) return rc;
+        memcpy(&total, w, sizeof(total));
     }
     L->count = (int64_t)std::min<unsigned long long>((unsigned long long)L->capacity, total);
-    return PBG_OK;
-}
-
-// One forward + backward pass on B rows of X (bf16 [B x 112]) with labels
-// Y; gradients into G1/G2/G3, gb1/gb2/gb3 (FP32); loss / correct in acc.
-// tc_gemm with its launches counted: the GEMM, and the split-K reduction
-// when a work buffer spreads K over slices.
-static int gemm(pbg_scene* s, const uint16_t* A, const uint16_t* B, float* C, int M, int N, int K, int acc,
-                int* status, cudaStream_t st, float* work) {
-    const int rc = tc_gemm(A, B, C, M, N, K, acc, status, st, work);
-    if (rc == PBG_OK)
-        s->counters.kernel_launches += 1 + (work && tc_gemm_work_floats(M, N, K) > (size_t)M * (size_t)N ? 1 : 0);
-    return rc;
-}
-
-static int forward_backward(pbg_scene* s, Learner* L, const uint16_t* X, const int32_t* Y, int B,
-                            cudaStream_t st) {
-    int* status = (int*)s->err.ptr;
-    int rc;
-    const size_t b = (size_t)B;
-    if ((rc = ensure(L->XT, b * kFeat * 2)) || (rc = ensure(L->Z1, b * kHidden * 4)) ||
-        (rc = ensure(L->Z2, b * kHidden * 4)) || (rc = ensure(L->Z3, b * kClusters * 4)) ||
-        (rc = ensure(L->H1, b * kHidden * 2)) || (rc = ensure(L->H2, b * kHidden * 2)) ||
-        (rc = ensure(L->H1T, b * kHidden * 2)) || (rc = ensure(L->H2T, b * kHidden * 2)) ||
-        (rc = ensure(L->dZ3, b * kClusters * 4)) || (rc = ensure(L->dZ3b, b * kClusters * 2)) ||
-        (rc = ensure(L->dZ3T, b * kClusters * 2)) || (rc = ensure(L->dH2, b * kHidden * 4)) ||
-        (rc = ensure(L->dZ2b, b * kHidden * 2)) || (rc = ensure(L->dZ2T, b * 128 * 2)) ||
-        (rc = ensure(L->dH1, b * kHidden * 4)) || (rc = ensure(L->dZ1b, b * kHidden * 2)) ||
-        (rc = ensure(L->dZ1T, b * 128 * 2)) || (rc = ensure(L->G1, 128 * kFeat * 4)) ||
-        (rc = ensure(L->G2, 128 * kHidden * 4)) || (rc = ensure(L->G3, kClusters * kHidden * 4)) ||
-        (rc = ensure(L->gb1, kHidden * 4)) || (rc = ensure(L->gb2, kHidden * 4)) ||
-        (rc = ensure(L->gb3, kClusters * 4)) || (rc = ensure(L->acc, 64)))
-        return rc;
-    {  // split-K workspace of the weight gradients (K = the batch)
-        const size_t wf = std::max({tc_gemm_work_floats(kClusters, kHidden, B),
-                                    tc_gemm_work_floats(128, kHidden, B), tc_gemm_work_floats(128, kFeat, B)});
-        if ((rc = ensure(L->gemm_work, wf * 4))) return rc;
-    }
-    auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
-    // forward
-    if ((rc = gemm(s, X, (const uint16_t*)L->W1b.ptr, (float*)L->Z1.ptr, B, kHidden, kFeat, 0, status, st, nullptr))) return rc;
-    bias_relu_kernel<<<blocks(b * kHidden), 256, 0, st>>>((float*)L->Z1.ptr, (const float*)L->b1.ptr, B, kHidden, 1,
-                                                           (uint16_t*)L->H1.ptr);
-    if ((rc = gemm(s, (const uint16_t*)L->H1.ptr, (const uint16_t*)L->W2b.ptr, (float*)L->Z2.ptr, B, kHidden,
-                      kHidden, 0, status, st, nullptr))) return rc;
-    bias_relu_kernel<<<blocks(b * kHidden), 256, 0, st>>>((float*)L->Z2.ptr, (const float*)L->b2.ptr, B, kHidden, 1,
-                                                           (uint16_t*)L->H2.ptr);
-    if ((rc = gemm(s, (const uint16_t*)L->H2.ptr, (const uint16_t*)L->W3b.ptr, (float*)L->Z3.ptr, B, kClusters,
-                      kHidden, 0, status, st, nullptr))) return rc;
-    bias_relu_kernel<<<blocks(b * kClusters), 256, 0, st>>>((float*)L->Z3.ptr, (const float*)L->b3.ptr, B,
-                                                             kClusters, 0, nullptr);
-    PBG_CUDA(cudaMemsetAsync(L->acc.ptr, 0, 8, st));
-    softmax_grad_kernel<<<(unsigned)((b * 32 + 255) / 256), 256, 0, st>>>(
-        (const float*)L->Z3.ptr, Y, B, B, 1.f / (float)B, (float*)L->dZ3.ptr, (uint16_t*)L->dZ3b.ptr,
-        (float*)L->acc.ptr);
-    // backward: dW3 = dZ3^T H2
-    transpose_bf16_kernel<<<blocks(b * kClusters), 256, 0, st>>>((const uint16_t*)L->dZ3b.ptr, B, kClusters,
-                                                                  kClusters, (uint16_t*)L->dZ3T.ptr);
-    transpose_bf16_kernel<<<blocks(b * kHidden), 256, 0, st>>>((const uint16_t*)L->H2.ptr, B, kHidden, kHidden,
-                                                                (uint16_t*)L->H2T.ptr);
-    if ((rc = gemm(s, (const uint16_t*)L->dZ3T.ptr, (const uint16_t*)L->H2T.ptr, (float*)L->G3.ptr, kClusters,
-                      kHidden, B, 0, status, st, (float*)L->gemm_work.ptr))) return rc;
-    colsum_kernel<<<kClusters, 256, 0, st>>>((const float*)L->dZ3.ptr, B, kClusters, (float*)L->gb3.ptr);
-    // dH2 = dZ3 W3 ; dZ2 = dH2 * relu'
-    if ((rc = gemm(s, (const uint16_t*)L->dZ3b.ptr, (const uint16_t*)L->W3Tb.ptr, (float*)L->dH2.ptr, B, kHidden,
-                      kClusters, 0, status, st, nullptr))) return rc;
-    relu_grad_kernel<<<blocks(b * kHidden), 256, 0, st>>>((float*)L->dH2.ptr, (const float*)L->Z2.ptr, b * kHidden,
-                                                           (uint16_t*)L->dZ2b.ptr);
-    colsum_kernel<<<kHidden, 256, 0, st>>>((const float*)L->dH2.ptr, B, kHidden, (float*)L->gb2.ptr);
-    // dW2 = dZ2^T H1 (rows padded to 128)
-    transpose_bf16_kernel<<<blocks(b * 128), 256, 0, st>>>((const uint16_t*)L->dZ2b.ptr, B, kHidden, 128,
-                                                            (uint16_t*)L->dZ2T.ptr);
-    transpose_bf16_kernel<<<blocks(b * kHidden), 256, 0, st>>>((const uint16_t*)L->H1.ptr, B, kHidden, kHidden,
-                                                                (uint16_t*)L->H1T.ptr);
-    if ((rc = gemm(s, (const uint16_t*)L->dZ2T.ptr, (const uint16_t*)L->H1T.ptr, (float*)L->G2.ptr, 128, kHidden,
-                      B, 0, status, st, (float*)L->gemm_work.ptr))) return rc;
-    // dH1 = dZ2 W2 ; dZ1 = dH1 * relu'
-    if ((rc = gemm(s, (const uint16_t*)L->dZ2b.ptr, (const uint16_t*)L->W2Tb.ptr, (float*)L->dH1.ptr, B, kHidden,
-                      kHidden, 0, status, st, nullptr))) return rc;
-    relu_grad_kernel<<<blocks(b * kHidden), 256, 0, st>>>((float*)L->dH1.ptr, (const float*)L->Z1.ptr, b * kHidden,
-                                                           (uint16_t*)L->dZ1b.ptr);
-    colsum_kernel<<<kHidden, 256, 0, st>>>((const float*)L->dH1.ptr, B, kHidden, (float*)L->gb1.ptr);
-    // dW1 = dZ1^T X (rows padded to 128)
-    transpose_bf16_kernel<<<blocks(b * 128), 256, 0, st>>>((const uint16_t*)L->dZ1b.ptr, B, kHidden, 128,
-                                                            (uint16_t*)L->dZ1T.ptr);
-    transpose_bf16_kernel<<<blocks(b * kFeat), 256, 0, st>>>(X, B, kFeat, kFeat, (uint16_t*)L->XT.ptr);
-    if ((rc = gemm(s, (const uint16_t*)L->dZ1T.ptr, (const uint16_t*)L->XT.ptr, (float*)L->G1.ptr, 128, kFeat, B,
-                      0, status, st, (float*)L->gemm_work.ptr))) return rc;
-    PBG_CUDA(cudaGetLastError());
-    s->counters.kernel_launches += 15;  // bias/ReLU 3, softmax 1, transposes 6, column sums 3, ReLU grads 2
-    return PBG_OK;
-}
-
-static int sgd_update(Learner* L, cudaStream_t st) {
-    const float lr = L->lr, m = L->momentum;
-    auto blocks = [](size_t n) { return (unsigned)((n + 255) / 256); };
-    sgd_kernel<<<blocks(kHidden * kFeat), 256, 0, st>>>((float*)L->W1.ptr, (float*)L->V1.ptr, (const float*)L->G1.ptr,
-                                                         kHidden, 105, kFeat, lr, m, (uint16_t*)L->W1b.ptr, nullptr, 0);
-    sgd_kernel<<<blocks(kHidden * kHidden), 256, 0, st>>>((float*)L->W2.ptr, (float*)L->V2.ptr,
-                                                           (const float*)L->G2.ptr, kHidden, kHidden, kHidden, lr, m,
-                                                           (uint16_t*)L->W2b.ptr, (uint16_t*)L->W2Tb.ptr, kHidden);
-    sgd_kernel<<<blocks(kClusters * kHidden), 256, 0, st>>>((float*)L->W3.ptr, (float*)L->V3.ptr,
-                                                             (const float*)L->G3.ptr, kClusters, kHidden, kHidden, lr,
-                                                             m, (uint16_t*)L->W3b.ptr, (uint16_t*)L->W3Tb.ptr,
-                                                             kClusters);
-    sgd_bias_kernel<<<1, kHidden, 0, st>>>((float*)L->b1.ptr, (float*)L->vb1.ptr, (const float*)L->gb1.ptr, kHidden, lr, m);
-    sgd_bias_kernel<<<1, kHidden, 0, st>>>((float*)L->b2.ptr, (float*)L->vb2.ptr, (const float*)L->gb2.ptr, kHidden, lr, m);
-    sgd_bias_kernel<<<1, kClusters, 0, st>>>((float*)L->b3.ptr, (float*)L->vb3.ptr, (const float*)L->gb3.ptr, kClusters, lr, m);
-    PBG_CUDA(cudaGetLastError());
     return PBG_OK;
 }
 
@@ -868,36 +570,31 @@ int learn_train(pbg_scene* s, int steps, cudaStream_t st) {
     Learner* L = s->learn;
     if (!L || !L->enabled) return PBG_OK;
     if (steps <= 0) steps = L->steps_per_train;
-    int rc0 = records_available(L, st);
+    int rc0 = records_available(s, L, st);
     if (rc0) return rc0;
     if (L->count < L->batch) return PBG_OK;  // not enough records yet
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, st);
+    for (cudaEvent_t& e : L->train_ev)
+        if (!e) PBG_CUDA(cudaEventCreate(&e));
+    PBG_CUDA(cudaEventRecord(L->train_ev[0], st));
     const int64_t nb = L->count / L->batch;
     int rc = PBG_OK;
     for (int k = 0; k < steps && rc == PBG_OK; ++k) {
         const int64_t start = ((int64_t)(L->trained_steps % (uint64_t)nb)) * L->batch;
-        const uint16_t* X = (const uint16_t*)L->recX.ptr + start * kFeat;
-        const int32_t* Y = (const int32_t*)L->recY.ptr + start;
-        rc = forward_backward(s, L, X, Y, L->batch, st);
-        if (rc == PBG_OK) rc = sgd_update(L, st);
-        if (rc == PBG_OK) s->counters.kernel_launches += 6;
+        rc = train_step(s, L, (const uint16_t*)L->recX.ptr + start * kFeat, (const int32_t*)L->recY.ptr + start,
+                        L->batch, true, k > 0, st);
         ++L->trained_steps;
     }
-    cudaEventRecord(e1, st);
-    float acc[2] = {0.f, 0.f};
-    cudaMemcpyAsync(acc, L->acc.ptr, 8, cudaMemcpyDeviceToHost, st);
-    cudaStreamSynchronize(st);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    L->train_ms += ms;
+    if (rc) return rc;
+    PBG_CUDA(cudaEventRecord(L->train_ev[1], st));
+    int w[2] = {0, 0};
+    if ((rc = read_device_words(s, (const int*)L->acc.ptr, 2, w, st))) return rc;
+    float acc[2], ms = 0.f;
+    memcpy(acc, w, sizeof(acc));
+    if (cudaEventSynchronize(L->train_ev[1]) == cudaSuccess &&
+        cudaEventElapsedTime(&ms, L->train_ev[0], L->train_ev[1]) == cudaSuccess)
+        L->train_ms += ms;
     L->last_loss = acc[0] / (float)L->batch;
     L->last_acc = acc[1] / (float)L->batch;
-    if (rc) return rc;
     return check_device_status(s, st);
 }
 
@@ -929,7 +626,7 @@ int pbg_learn_get_stats(pbg_scene* s, pbg_learn_stats* out) {
     memset(out, 0, sizeof(*out));
     if (!L) return PBG_OK;
     cudaSetDevice(s->device);
-    int rc = records_available(L, s->stream);
+    int rc = records_available(s, L, s->stream);
     if (rc) return rc;
     out->trained_steps = L->trained_steps;
     out->records = (uint64_t)L->count;
@@ -945,24 +642,11 @@ int pbg_learn_params_io(pbg_scene* s, float* params, int32_t get) {
     if (!s || !params || !s->learn) return PBG_ERR_INVALID_ARGUMENT;
     cudaSetDevice(s->device);
     Learner* L = s->learn;
-    const size_t n1 = (size_t)kHidden * kFeat, n2 = (size_t)kHidden * kHidden, n3 = (size_t)kClusters * kHidden;
-    float* p = params;
     if (get) {
-        PBG_CUDA(cudaMemcpy(p, L->W1.ptr, n1 * 4, cudaMemcpyDeviceToHost)); p += n1;
-        PBG_CUDA(cudaMemcpy(p, L->b1.ptr, kHidden * 4, cudaMemcpyDeviceToHost)); p += kHidden;
-        PBG_CUDA(cudaMemcpy(p, L->W2.ptr, n2 * 4, cudaMemcpyDeviceToHost)); p += n2;
-        PBG_CUDA(cudaMemcpy(p, L->b2.ptr, kHidden * 4, cudaMemcpyDeviceToHost)); p += kHidden;
-        PBG_CUDA(cudaMemcpy(p, L->W3.ptr, n3 * 4, cudaMemcpyDeviceToHost)); p += n3;
-        PBG_CUDA(cudaMemcpy(p, L->b3.ptr, kClusters * 4, cudaMemcpyDeviceToHost));
+        PBG_CUDA(cudaMemcpy(params, L->P.ptr, kParams * 4, cudaMemcpyDeviceToHost));
         return PBG_OK;
     }
-    std::vector<float> w1(p, p + n1); p += n1;
-    std::vector<float> b1(p, p + kHidden); p += kHidden;
-    std::vector<float> w2(p, p + n2); p += n2;
-    std::vector<float> b2(p, p + kHidden); p += kHidden;
-    std::vector<float> w3(p, p + n3); p += n3;
-    std::vector<float> b3(p, p + kClusters);
-    return upload_params(L, w1, b1, w2, b2, w3, b3, s->stream);
+    return upload_params(L, params, s->stream);
 }
 
 int pbg_learn_gradients(pbg_scene* s, const float* x, const int32_t* labels, int32_t B, float* grads,
@@ -982,15 +666,8 @@ int pbg_learn_gradients(pbg_scene* s, const float* x, const int32_t* labels, int
     if ((rc = ensure(L->X, xb.size() * 2)) || (rc = ensure(L->feat, (size_t)B * 4))) return rc;
     PBG_CUDA(cudaMemcpyAsync(L->X.ptr, xb.data(), xb.size() * 2, cudaMemcpyHostToDevice, st));
     PBG_CUDA(cudaMemcpyAsync(L->feat.ptr, labels, (size_t)B * 4, cudaMemcpyHostToDevice, st));
-    if ((rc = forward_backward(s, L, (const uint16_t*)L->X.ptr, (const int32_t*)L->feat.ptr, B, st))) return rc;
-    const size_t n1 = (size_t)kHidden * kFeat, n2 = (size_t)kHidden * kHidden, n3 = (size_t)kClusters * kHidden;
-    float* g = grads;
-    PBG_CUDA(cudaMemcpyAsync(g, L->G1.ptr, n1 * 4, cudaMemcpyDeviceToHost, st)); g += n1;  // first 64 rows
-    PBG_CUDA(cudaMemcpyAsync(g, L->gb1.ptr, kHidden * 4, cudaMemcpyDeviceToHost, st)); g += kHidden;
-    PBG_CUDA(cudaMemcpyAsync(g, L->G2.ptr, n2 * 4, cudaMemcpyDeviceToHost, st)); g += n2;
-    PBG_CUDA(cudaMemcpyAsync(g, L->gb2.ptr, kHidden * 4, cudaMemcpyDeviceToHost, st)); g += kHidden;
-    PBG_CUDA(cudaMemcpyAsync(g, L->G3.ptr, n3 * 4, cudaMemcpyDeviceToHost, st)); g += n3;
-    PBG_CUDA(cudaMemcpyAsync(g, L->gb3.ptr, kClusters * 4, cudaMemcpyDeviceToHost, st));
+    if ((rc = train_step(s, L, (const uint16_t*)L->X.ptr, (const int32_t*)L->feat.ptr, B, false, false, st))) return rc;
+    PBG_CUDA(cudaMemcpyAsync(grads, L->G.ptr, kParams * 4, cudaMemcpyDeviceToHost, st));
     float acc[2];
     PBG_CUDA(cudaMemcpyAsync(acc, L->acc.ptr, 8, cudaMemcpyDeviceToHost, st));
     PBG_CUDA(cudaStreamSynchronize(st));

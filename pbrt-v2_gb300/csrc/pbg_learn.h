@@ -11,13 +11,21 @@ constexpr int kFeat = 112;      // 105 features padded to a multiple of 16
 constexpr int kHidden = 64;
 constexpr int kClusters = 256;
 
+// The parameters as one array, in the order of pbg_learn_params_io: W1 [64 x
+// 112], b1, W2 [64 x 64], b2, W3 [256 x 64], b3.
+constexpr int kOffW1 = 0, kOffB1 = kHidden * kFeat, kOffW2 = kOffB1 + kHidden, kOffB2 = kOffW2 + kHidden * kHidden,
+              kOffW3 = kOffB2 + kHidden, kOffB3 = kOffW3 + kClusters * kHidden, kParams = kOffB3 + kClusters;
+// A CTA's partial gradient: the parameters' order, then its loss and number
+// of right answers; rows start on 16 bytes.
+constexpr int kPartFloats = (kParams + 2 + 3) / 4 * 4;
+
 struct LearnBox {
     float lo[3], inv_ext[3];
 };
 
-// Device buffers of one learner.  W*: FP32 master weights [out x in_pad],
-// V*: momentum, Wb*: BF16 [out x in_pad] (forward), WTb*: BF16 [in x out]
-// (backward dH), b*: biases.
+// Device buffers of one learner.  P: FP32 master parameters, V: their
+// momentum, Wb: their BF16 copies (weights only are read), G: gradients
+// (pbg_learn_gradients), part: the CTAs' partial gradients.
 struct Learner {
     bool enabled = false;
     int batch = 8192;
@@ -36,11 +44,8 @@ struct Learner {
     int nclusters = 0;
     bool clusters_built = false;
     DeviceBuffer occ_prim;  // any-hit batches: the occluder each walk found
-    // parameters
-    DeviceBuffer W1, W2, W3, V1, V2, V3, b1, b2, b3, vb1, vb2, vb3, W1b, W2b, W3b, W2Tb, W3Tb;
-    // training scratch
-    DeviceBuffer recX, recY, X, XT, Z1, Z2, Z3, H1, H2, H1T, H2T, dZ3, dZ3b, dZ3T, dH2, dZ2b, dZ2T,
-        dH1, dZ1b, dZ1T, G1, G2, G3, gb1, gb2, gb3, acc, gemm_work;
+    DeviceBuffer P, V, Wb, G, part, acc;
+    DeviceBuffer recX, recY, X;
     // per-batch inference scratch
     DeviceBuffer feat, pred;
     float last_loss = 0.f, last_acc = 0.f;
@@ -48,6 +53,7 @@ struct Learner {
     // event pairs around inference launches, summed into infer_ms when the
     // statistics are read (no synchronisation on the launch path)
     std::vector<cudaEvent_t> infer_ev, infer_pool;
+    cudaEvent_t train_ev[2] = {};
 };
 
 int learn_init(pbg_scene* s, const pbg_learn_params* p);
@@ -68,5 +74,11 @@ int learn_predict(pbg_scene* s, const float4* o, const float4* d, int64_t n, con
 int learn_collect(pbg_scene* s, const float4* o, const float4* d, const int32_t* prim, int64_t n,
                   cudaStream_t st);
 int learn_train(pbg_scene* s, int steps, cudaStream_t st);
+// Forward and backward pass on B records (B % 128 == 0) of X (bf16 [B x 112])
+// with labels Y; then the SGD step (update), or the gradients into G.  The
+// batch's loss sum and number of right answers go to acc[0..1].  chained:
+// the previous launch on st was another train_step of the same call.
+int train_step(pbg_scene* s, Learner* L, const uint16_t* X, const int32_t* Y, int B, bool update, bool chained,
+               cudaStream_t st);
 
 }  // namespace pbg

@@ -97,6 +97,33 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// Two runs of eight columns (v[0-7] and v[8-15]), read or written.
+__device__ __forceinline__ void tmem_ld8x2(uint32_t t0, uint32_t t1, float* v) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(t0), "r"(t1)
+        : "memory");
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+}
+__device__ __forceinline__ void tmem_st8x2(uint32_t t0, uint32_t t1, const float* v) {
+    uint32_t r[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) r[k] = __float_as_uint(v[k]);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%2,%3,%4,%5,%6,%7,%8,%9};\n\t"
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%1], {%10,%11,%12,%13,%14,%15,%16,%17};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(t0),
+        "r"(t1), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+
 __device__ __forceinline__ uint16_t f2bf(float x) {
     // round to nearest even (inputs here are finite)
     uint32_t u = __float_as_uint(x);
@@ -104,6 +131,19 @@ __device__ __forceinline__ uint16_t f2bf(float x) {
     return (uint16_t)(u >> 16);
 }
 __device__ __forceinline__ float bf2f(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
+
+// Two values rounded to nearest even in one word, the first in the lower
+// half (f2bf twice, in one instruction).
+__device__ __forceinline__ uint32_t f2bf2(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+
+// Eight values as bf16 in one 16-byte word (a core-matrix row).
+__device__ __forceinline__ uint4 pack8(const float* v) {
+    return make_uint4(f2bf2(v[0], v[1]), f2bf2(v[2], v[3]), f2bf2(v[4], v[5]), f2bf2(v[6], v[7]));
+}
 
 #endif  // __CUDACC__
 
