@@ -899,8 +899,7 @@ __global__ void gather_mesh_kernel(const float* __restrict__ P, const int32_t* _
 }
 
 // The scene's accelerator structures from triangles already in s->tri9 on
-// the device: naive needs only the records; ray-bvh builds its tree on the
-// device.  (rayhierarchy orders its records on the host; see scene_build.)
+// the device: naive orders its records into groups; ray-bvh builds its tree.  (rayhierarchy orders its records on the host; see scene_build.)
 static int scene_build_device(pbg_scene* s) {
     const int64_t ntri = s->ntri;
     const size_t nt = (size_t)(ntri > 0 ? ntri : 1);
@@ -916,17 +915,10 @@ static int scene_build_device(pbg_scene* s) {
             return rc;
         }
     } else {
-        // scene bounds for the naive scene (the device builder computes them for ray-bvh)
-        std::vector<float> h((size_t)ntri * 9);
-        if (ntri > 0) PBG_CUDA(cudaMemcpy(h.data(), s->tri9.ptr, h.size() * 4, cudaMemcpyDeviceToHost));
-        for (int64_t i = 0; i < ntri; ++i)
-            for (int k = 0; k < 9; ++k) {
-                const float v = h[9 * i + k];
-                const int a = k % 3;
-                if (i == 0 && k < 3) s->scene_lo[a] = s->scene_hi[a] = v;
-                s->scene_lo[a] = v < s->scene_lo[a] ? v : s->scene_lo[a];
-                s->scene_hi[a] = v > s->scene_hi[a] ? v : s->scene_hi[a];
-            }
+        if ((rc = naive_build(s, order))) {
+            release(order);
+            return rc;
+        }
     }
     if (ntri > 0) {
         build_tris_kernel<<<(unsigned)((ntri + 255) / 256), 256, 0, s->stream>>>(
@@ -1148,6 +1140,8 @@ void pbg_scene_destroy(pbg_scene* s) {
     release(s->bvh);
     release(s->wide);
     release(s->tris_wide);
+    release(s->naive_groups);
+    release(s->naive_normals);
     release(s->spheres);
     release(s->clusters);
     release(s->tri_pos);

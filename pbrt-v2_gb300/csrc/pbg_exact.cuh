@@ -128,7 +128,12 @@ __device__ __forceinline__ bool pbg_filter(const TriRec& tr, float4 o, float4 d,
     float ediv = fmaf(ck, ne1, kFilterTiny);  // bound on |div_f - div_ref|
     float e1b = fmaf(ck, nv, kFilterTiny);    // bound on |n1_f - n1_ref|
     float D = fabsf(div);
-    if (!(D > ediv)) return true;  // sign of the divisor (or zero) uncertain
+    if (!(D > ediv))
+        // The divisor's sign (or zero) is uncertain, but it is at most D +
+        // ediv: a numerator above that makes |b1| > 1, rejected by either
+        // sign's check (a zero divisor is rejected anyway).  This settles
+        // nearly every test of a degenerate triangle, which every ray makes.
+        return !(fabsf(n1) - e1b > (D + ediv) * (1.f + 2.f * kFilterR));
     float a1 = flip_sign(n1, div);
     float top = fmaf(D, 1.f + kFilterR, ediv);
     if (a1 < -e1b || a1 > top + e1b) return false;
@@ -153,9 +158,10 @@ __device__ __forceinline__ bool pbg_filter(const TriRec& tr, float4 o, float4 d,
 
 // Orderable key for a nearest hit: larger key = nearer hit; equal t -> larger
 // triangle index, which is the answer of pbrt's in-order loop (equal t is
-// accepted again, so the last index wins).  0 = no hit.
+// accepted again, so the last index wins; -0 equals +0 there and here).  0 =
+// no hit.
 __device__ __forceinline__ unsigned long long hit_key(float t, int32_t prim) {
-    uint32_t b = __float_as_uint(t);
+    uint32_t b = __float_as_uint(__fadd_rn(t, 0.f));  // -0 -> +0
     uint32_t ord = (b & 0x80000000u) ? ~b : (b | 0x80000000u);  // ascending in t
     return ((unsigned long long)(~ord) << 32) | (uint32_t)prim;
 }

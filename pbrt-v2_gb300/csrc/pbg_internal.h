@@ -76,7 +76,7 @@ constexpr int kClusterTris = 32;
 // Launch-shape settings that change no result, chosen by pbg_autotune (the
 // defaults are the shapes measured best on the benchmark scenes).
 struct Tunables {
-    int naive_ctas = 4;      // naive: CTAs per SM the triangle splits aim for
+    int naive_ctas = 16;     // naive: CTAs per SM the triangle splits aim for
     // rayhierarchy [any-hit]: nodes of the level the descent starts at (at
     // most), CTAs per SM of the grid-stride kernels
     int rh_seed[2] = {256, 256};
@@ -117,6 +117,8 @@ struct pbg_scene {
     int64_t wide_nodes = 0;
     std::vector<int32_t> bvh_levels;  // device-built tree: (first node, nodes) per level, root first
     int wide_state = 0;        // 0 not built yet, 1 built, -1 the tree does not fit the wide format
+    pbg::DeviceBuffer naive_groups; // NaiveGroup per 32 records past the unculled ones (naive)
+    pbg::DeviceBuffer naive_normals; // unit normal and longest edge per record (naive)
     pbg::DeviceBuffer spheres; // float4 bounding sphere per record (rayhierarchy)
     pbg::DeviceBuffer clusters; // float4 sphere per kClusterTris consecutive records (rayhierarchy)
     pbg::DeviceBuffer tri_pos; // original index -> record position
@@ -149,6 +151,9 @@ namespace pbg {
 // Kernel launchers (one translation unit each).
 int launch_pack_rays(pbg_scene* s, const float* stage, int64_t n, float4* o, float4* d,
                      cudaStream_t st);
+// Orders a naive scene's triangles (original order in s->tri9) into groups
+// that rays can skip: the record order into `order`, s->unculled, s->naive_groups.
+int naive_build(pbg_scene* s, DeviceBuffer& order);
 int naive_nearest(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
                   int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
 int naive_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,

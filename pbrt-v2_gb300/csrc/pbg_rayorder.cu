@@ -15,6 +15,7 @@
 // (2) one exclusive scan over [digit][tile] counts, (3) a stable scatter in
 // which each warp ranks its 32 keys per digit with __match_any_sync and the
 // tile's warps are combined through shared-memory prefix sums.
+#include "pbg_curve.cuh"
 #include "pbg_internal.h"
 #include "pbg_tma.cuh"
 
@@ -126,45 +127,6 @@ __global__ void morton_kernel(const float4* __restrict__ ro, const float4* __res
 // silhouette pixels' far-apart hit points together); unlike a Morton code,
 // consecutive cells of the curve are always neighbours, so no leaf spans a
 // jump.
-__device__ __forceinline__ uint32_t spread10(uint32_t v) {
-    v &= 0x3ffu;
-    v = (v | (v << 16)) & 0x030000ffu;
-    v = (v | (v << 8)) & 0x0300f00fu;
-    v = (v | (v << 4)) & 0x030c30c3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
-}
-
-// 3-D Hilbert index in transposed form (J. Skilling, "Programming the
-// Hilbert curve", AIP Conf. Proc. 707, 2004): the coordinates are rewritten
-// in place so that interleaving their bits, as for a Morton code, gives the
-// cell's position along the Hilbert curve, whose consecutive cells are
-// always face neighbours.
-__device__ __forceinline__ void hilbert3(uint32_t x[3], int bits) {
-    const uint32_t top = 1u << (bits - 1);
-    for (uint32_t q = top; q > 1; q >>= 1) {
-        const uint32_t p = q - 1;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (x[a] & q) {
-                x[0] ^= p;
-            } else {
-                const uint32_t t = (x[0] ^ x[a]) & p;
-                x[0] ^= t;
-                x[a] ^= t;
-            }
-        }
-    }
-    x[1] ^= x[0];
-    x[2] ^= x[1];
-    uint32_t t = 0;
-    for (uint32_t q = top; q > 1; q >>= 1)
-        if (x[2] & q) t ^= q - 1;
-    x[0] ^= t;
-    x[1] ^= t;
-    x[2] ^= t;
-}
-
 __global__ void origin_key_kernel(const float4* __restrict__ ro, const uint8_t* __restrict__ valid,
                                   int64_t n, const int* __restrict__ bounds, uint32_t* __restrict__ keys,
                                   int32_t* __restrict__ vals) {
@@ -430,6 +392,13 @@ __global__ void __launch_bounds__(kSortThreads)
     }
 }
 
+// Words of radix_sort_pairs' histogram buffer for n keys: the counts, eight
+// words for bounds, the scan's chunk sums.
+size_t radix_hist_words(int64_t n) {
+    const size_t m = (size_t)((n + kSortTile - 1) / kSortTile) * kRadix;
+    return m + 8 + (m + kScanChunk - 1) / kScanChunk + 8;
+}
+
 // Sorts (keys, vals) of length n in place through the tmp buffers; returns
 // pointers to the sorted arrays (which alternate between the two buffers).
 int radix_sort_pairs(pbg_scene* s, uint32_t* keys, int32_t* vals, uint32_t* keys_tmp, int32_t* vals_tmp,
@@ -507,8 +476,7 @@ int ray_sort(pbg_scene* s, const float4* o, const float4* d, const uint8_t* vali
     int rc;
     if ((rc = ensure(w.mkeys, (size_t)n * 4)) || (rc = ensure(w.mkeys_tmp, (size_t)n * 4)) ||
         (rc = ensure(w.perm, (size_t)n * 4)) || (rc = ensure(w.perm_tmp, (size_t)n * 4)) ||
-        (rc = ensure(w.hist, ((size_t)tiles * kRadix + 8 +
-                              ((size_t)tiles * kRadix + kScanChunk - 1) / kScanChunk + 8) * 4)))
+        (rc = ensure(w.hist, radix_hist_words(n) * 4)))
         return rc;
     int* bounds = (int*)((uint32_t*)w.hist.ptr + (size_t)tiles * kRadix);
     int sms = 152;
