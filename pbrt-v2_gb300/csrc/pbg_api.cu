@@ -98,6 +98,11 @@ __global__ void pack_rays_kernel(const float* __restrict__ stage, int64_t n, flo
 
 __device__ __forceinline__ void xcross3(float ax, float ay, float az, float bx, float by, float bz,
                                         float* x, float* y, float* z) {
+    bool ok = true;
+    *x = xcross_f32(ay, bz, az, by, ok);
+    *y = xcross_f32(az, bx, ax, bz, ok);
+    *z = xcross_f32(ax, by, ay, bx, ok);
+    if (ok) return;
     *x = xcross(ay, bz, az, by);
     *y = xcross(az, bx, ax, bz);
     *z = xcross(ax, by, ay, bx);

@@ -32,7 +32,8 @@ __global__ void __launch_bounds__(kBvhThreads, kBvhMinBlocks)
                int32_t* __restrict__ prim_out, float* __restrict__ t_out,
                float* __restrict__ b1_out, float* __restrict__ b2_out, uint8_t* __restrict__ occ,
                int* status, unsigned long long* wcount, const uint16_t* __restrict__ pred,
-               const int32_t* __restrict__ cref) {
+               const int32_t* __restrict__ cref, const uint32_t* __restrict__ n_dev) {
+    if (n_dev) n = *n_dev;
     const int64_t slot = (int64_t)blockIdx.x * kBvhThreads + threadIdx.x;
     if (slot >= n) return;
     const int64_t ray = perm ? (int64_t)perm[slot] : slot;
@@ -96,7 +97,8 @@ __global__ void __launch_bounds__(kPacketThreads)
                       const uint8_t* __restrict__ valid, const int32_t* __restrict__ perm, int64_t n,
                       int32_t* __restrict__ prim_out, float* __restrict__ t_out, float* __restrict__ b1_out,
                       float* __restrict__ b2_out, uint8_t* __restrict__ occ, int* status,
-                      unsigned long long* next, unsigned long long* wcount) {
+                      unsigned long long* next, unsigned long long* wcount, const uint32_t* __restrict__ n_dev) {
+    if (n_dev) n = *n_dev;
     __shared__ int32_t stk[kPacketThreads / 32][kPacketStack];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -209,7 +211,8 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
                           float* __restrict__ b1_out, float* __restrict__ b2_out,
                           uint8_t* __restrict__ occ, int* status, unsigned long long* next,
                           const uint16_t* __restrict__ pred, const int32_t* __restrict__ cref,
-                          unsigned long long* wcount) {
+                          unsigned long long* wcount, const uint32_t* __restrict__ n_dev) {
+    if (n_dev) n = *n_dev;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
@@ -400,6 +403,36 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
 int ray_order(pbg_scene* s, const float4* o, const float4* d, int64_t n, const int32_t** perm,
               cudaStream_t st);
 
+// The counter that a persistent walk's warps take rays from: the caller's, or
+// the scene's own, zeroed.
+static int walk_counter(pbg_scene* s, const QueueRef& q, unsigned long long** next, cudaStream_t st) {
+    *next = q.next;
+    if (q.next) return PBG_OK;
+    const int rc = ensure(s->work.counters, 64);
+    if (rc) return rc;
+    *next = (unsigned long long*)s->work.counters.ptr;
+    PBG_CUDA(cudaMemsetAsync(*next, 0, sizeof(unsigned long long), st));
+    return PBG_OK;
+}
+
+// The walk of a batch class (hint 1: incoherent).
+static int choose_walk(const pbg_scene* s, bool any, int hint) {
+    if (s->params.walk != 0) return s->params.walk;
+    const int tuned = s->tune.bvh_walk[any ? 1 : 0][hint == 1 ? 1 : 0];
+    if (tuned != 0) return tuned;
+    // untuned: the walks the autotuner picked on both benchmark scenes' batch
+    // classes (camera rays 4; their shadow rays 5; bounce rays and their
+    // shadows 6), none of them more than 25 % off the class's best there
+    return hint == 1 ? 6 : (any ? 5 : 4);
+}
+
+// Walk 3 sorts the batch and the learned ordering records it, both for a
+// length known to the host.
+bool bvh_queue_ok(const pbg_scene* s) {
+    if (s->params.ray_sort > 0 || (s->learn && s->learn->enabled)) return false;
+    return choose_walk(s, false, 1) != 3 && choose_walk(s, true, 0) != 3 && choose_walk(s, true, 1) != 3;
+}
+
 // cluster_hint: a caller's cluster per ray (kNoCluster or any value outside
 // 0..kClusters-1 = none), walked first; else
 // the learned ordering's prediction when it is on for this kind of query.
@@ -407,7 +440,7 @@ int ray_order(pbg_scene* s, const float4* o, const float4* d, int64_t n, const i
 template <bool ANY>
 static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid,
                       int64_t n, int32_t* prim, float* t, float* b1, float* b2, uint8_t* occ,
-                      const uint16_t* cluster_hint, int32_t* occluders, cudaStream_t st) {
+                      const uint16_t* cluster_hint, int32_t* occluders, cudaStream_t st, QueueRef q = QueueRef()) {
     if (n <= 0) return PBG_OK;
     const int32_t* perm = nullptr;
     if (s->params.ray_sort > 0) {
@@ -441,12 +474,7 @@ static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint
     // bounce batches are incoherent: the reference's bounce form of Intersect
     // is the one with a validity mask (rayhierarchy.cpp:602-813)
     const int hint = s->walk_hint >= 0 ? s->walk_hint : (!ANY && valid != nullptr ? 1 : 0);
-    const int tuned = s->tune.bvh_walk[ANY ? 1 : 0][hint == 1 ? 1 : 0];
-    // untuned: the walks the autotuner picked on both benchmark scenes' batch
-    // classes (camera rays 4; their shadow rays 5; bounce rays and their
-    // shadows 6), none of them more than 25 % off the class's best there
-    const int fallback = hint == 1 ? 6 : (ANY ? 5 : 4);
-    int walk = s->params.walk != 0 ? s->params.walk : (tuned != 0 ? tuned : fallback);
+    int walk = choose_walk(s, ANY, hint);
     // Host-buffer calls run the packets in the caller's order: there the
     // batch arrives in parts whose copies overlap the traversal, and sorting
     // each part cost more than its packets gained (terrain frame end to end:
@@ -476,11 +504,8 @@ static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint
     }
     prof_begin(s, st);
     if (packet) {
-        int rc3 = PBG_OK;
-        Work& w = s->work;
-        if ((rc3 = ensure(w.counters, 64))) return rc3;
-        unsigned long long* next = (unsigned long long*)w.counters.ptr;
-        PBG_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+        unsigned long long* next = nullptr;
+        if ((rc = walk_counter(s, q, &next, st))) return rc;
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh_packet_kernel<ANY, false>, kPacketThreads, 0);
         int sms = 152;
@@ -490,18 +515,15 @@ static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint
         const bool stats = s->prof.level >= 2;
         auto kern = stats ? bvh_packet_kernel<ANY, true> : bvh_packet_kernel<ANY, false>;
         kern<<<(unsigned)blocks, kPacketThreads, 0, st>>>(nodes, tris, s->unculled, o, d, valid, order, n, prim, t,
-                                                          b1, b2, occ, status, next, stats ? wc : nullptr);
+                                                          b1, b2, occ, status, next, stats ? wc : nullptr, q.n_dev);
     } else if (wide) {
-        rc = ANY ? wide_occluded(s, walk == 6, o, d, valid, perm, n, prim, occ, st)
-                 : wide_nearest(s, walk == 6, o, d, valid, perm, n, prim, t, b1, b2, st);
+        rc = ANY ? wide_occluded(s, walk == 6, o, d, valid, perm, n, q, prim, occ, st)
+                 : wide_nearest(s, walk == 6, o, d, valid, perm, n, q, prim, t, b1, b2, st);
         if (rc) return rc;
     } else if (persistent) {
         // persistent while-while walk: one counter word, zeroed per launch
-        Work& w = s->work;
-        int rc2 = ensure(w.counters, 64);
-        if (rc2) return rc2;
-        unsigned long long* next = (unsigned long long*)w.counters.ptr;
-        PBG_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+        unsigned long long* next = nullptr;
+        if ((rc = walk_counter(s, q, &next, st))) return rc;
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bvh_persistent_kernel<ANY, false, false, true>,
                                                       kPersistThreads, 0);
@@ -522,24 +544,24 @@ static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint
                                           : bvh_persistent_kernel<ANY, false, false, false>));
         kern<<<(unsigned)blocks, kPersistThreads, 0, st>>>(nodes, tris, s->unculled, o, d, valid, perm, n,
                                                            prim, t, b1, b2, occ, status, next, pred, cref,
-                                                           stats ? wc : nullptr);
+                                                           stats ? wc : nullptr, q.n_dev);
     } else if (pred) {
         if (s->prof.level >= 2)
             bvh_kernel<ANY, true, true><<<grid, kBvhThreads, 0, st>>>(
-                nodes, tris, s->unculled, o, d, valid, perm, n, prim, t, b1, b2, occ, status, wc, pred, cref);
+                nodes, tris, s->unculled, o, d, valid, perm, n, prim, t, b1, b2, occ, status, wc, pred, cref, q.n_dev);
         else
             bvh_kernel<ANY, false, true><<<grid, kBvhThreads, 0, st>>>(
                 nodes, tris, s->unculled, o, d, valid, perm, n, prim, t, b1, b2, occ, status, nullptr, pred,
-                cref);
+                cref, q.n_dev);
     } else {
         if (s->prof.level >= 2)
             bvh_kernel<ANY, true, false><<<grid, kBvhThreads, 0, st>>>(
                 nodes, tris, s->unculled, o, d, valid, perm, n, prim, t, b1, b2, occ, status, wc, nullptr,
-                nullptr);
+                nullptr, q.n_dev);
         else
             bvh_kernel<ANY, false, false><<<grid, kBvhThreads, 0, st>>>(
                 nodes, tris, s->unculled, o, d, valid, perm, n, prim, t, b1, b2, occ, status, nullptr,
-                nullptr, nullptr);
+                nullptr, nullptr, q.n_dev);
     }
     prof_end(s, st, kStageTraverse, 1);
     PBG_CUDA(cudaGetLastError());
@@ -556,6 +578,17 @@ int bvh_nearest(pbg_scene* s, const float4* o, const float4* d, const uint8_t* v
 int bvh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
                  uint8_t* occ, cudaStream_t st) {
     return bvh_launch<true>(s, o, d, valid, n, nullptr, nullptr, nullptr, nullptr, occ, nullptr, nullptr, st);
+}
+
+int bvh_queue_nearest(pbg_scene* s, const float4* o, const float4* d, int64_t n, const uint32_t* n_dev,
+                      unsigned long long* next, int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st) {
+    return bvh_launch<false>(s, o, d, nullptr, n, prim, t, b1, b2, nullptr, nullptr, nullptr, st, QueueRef{n_dev, next});
+}
+
+int bvh_queue_occluded(pbg_scene* s, const float4* o, const float4* d, int64_t n, const uint32_t* n_dev,
+                       unsigned long long* next, uint8_t* occ, cudaStream_t st) {
+    return bvh_launch<true>(s, o, d, nullptr, n, nullptr, nullptr, nullptr, nullptr, occ, nullptr, nullptr, st,
+                            QueueRef{n_dev, next});
 }
 
 int bvh_nearest_hinted(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,

@@ -30,8 +30,13 @@ __device__ __forceinline__ V3 vmul(V3 a, float s) {
 }
 __device__ __forceinline__ V3 vneg(V3 a) { return V3{-a.x, -a.y, -a.z}; }
 __device__ __forceinline__ float vdot(V3 a, V3 b) { return xdot(a.x, a.y, a.z, b.x, b.y, b.z); }
+// pbrt's Cross: the FP32 form with its proof of the double rounding, FP64
+// (a small fraction of FP32's rate) only where the proof fails.
 __device__ __forceinline__ V3 vcross(V3 a, V3 b) {
-    return V3{xcross(a.y, b.z, a.z, b.y), xcross(a.z, b.x, a.x, b.z), xcross(a.x, b.y, a.y, b.x)};
+    bool ok = true;
+    V3 c{xcross_f32(a.y, b.z, a.z, b.y, ok), xcross_f32(a.z, b.x, a.x, b.z, ok), xcross_f32(a.x, b.y, a.y, b.x, ok)};
+    if (!ok) c = V3{xcross(a.y, b.z, a.z, b.y), xcross(a.z, b.x, a.x, b.z), xcross(a.x, b.y, a.y, b.x)};
+    return c;
 }
 __device__ __forceinline__ float vlen(V3 a) { return __fsqrt_rn(vdot(a, a)); }
 __device__ __forceinline__ V3 vnormalize(V3 a) { return vmul(a, __frcp_rn(vlen(a))); }

@@ -166,6 +166,21 @@ int bvh_nearest_hinted(pbg_scene* s, const float4* o, const float4* d, const uin
                        const uint16_t* hint, int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
 int bvh_occluded_hinted(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
                         const uint16_t* hint, uint8_t* occ, int32_t* occluders, cudaStream_t st);
+// Batches whose length the host does not know (a renderer's bounce queues):
+// n is its upper bound, *n_dev the length, *next a walk counter of the
+// caller's, zero before the launch.  bvh_queue_ok: every class of the frame's
+// batches has a walk that can be launched so.
+bool bvh_queue_ok(const pbg_scene* s);
+int bvh_queue_nearest(pbg_scene* s, const float4* o, const float4* d, int64_t n, const uint32_t* n_dev,
+                      unsigned long long* next, int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
+int bvh_queue_occluded(pbg_scene* s, const float4* o, const float4* d, int64_t n, const uint32_t* n_dev,
+                       unsigned long long* next, uint8_t* occ, cudaStream_t st);
+// A batch's length and walk counter on the device (both NULL: n rays, the
+// scene's own counter).
+struct QueueRef {
+    const uint32_t* n_dev = nullptr;
+    unsigned long long* next = nullptr;
+};
 // Walks 5 and 6 (coop) over the eight-wide tree; ensure_wide builds it on
 // first use and sets *available = false when the scene keeps the two-wide
 // walks.
@@ -176,9 +191,10 @@ int ensure_wide(pbg_scene* s, bool* available, cudaStream_t st);
 // tree does not fit the wide format.
 int collapse_wide_device(pbg_scene* s, bool* fits, DeviceBuffer& src, int64_t* nwide, cudaStream_t st);
 int wide_nearest(pbg_scene* s, bool coop, const float4* o, const float4* d, const uint8_t* valid,
-                 const int32_t* perm, int64_t n, int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
+                 const int32_t* perm, int64_t n, QueueRef q, int32_t* prim, float* t, float* b1, float* b2,
+                 cudaStream_t st);
 int wide_occluded(pbg_scene* s, bool coop, const float4* o, const float4* d, const uint8_t* valid,
-                  const int32_t* perm, int64_t n, int32_t* occluders, uint8_t* occ, cudaStream_t st);
+                  const int32_t* perm, int64_t n, QueueRef q, int32_t* occluders, uint8_t* occ, cudaStream_t st);
 int rh_nearest(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
                int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
 int rh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,

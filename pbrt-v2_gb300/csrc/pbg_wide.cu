@@ -444,12 +444,14 @@ int ensure_wide(pbg_scene* s, bool* available, cudaStream_t st) {
 
 template <bool ANY, bool COOP>
 int wide_launch(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, const int32_t* perm,
-                int64_t n, int32_t* prim, float* t, float* b1, float* b2, uint8_t* occ, cudaStream_t st) {
-    Work& w = s->work;
-    int rc = ensure(w.counters, 64);
-    if (rc) return rc;
-    unsigned long long* next = (unsigned long long*)w.counters.ptr;
-    PBG_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+                int64_t n, QueueRef q, int32_t* prim, float* t, float* b1, float* b2, uint8_t* occ, cudaStream_t st) {
+    unsigned long long* next = q.next;
+    if (!next) {
+        const int rc = ensure(s->work.counters, 64);
+        if (rc) return rc;
+        next = (unsigned long long*)s->work.counters.ptr;
+        PBG_CUDA(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
+    }
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wide_walk_kernel<ANY, false, COOP, SceneRays>, kWideThreads, 0);
     int sms = 152;
@@ -458,7 +460,7 @@ int wide_launch(pbg_scene* s, const float4* o, const float4* d, const uint8_t* v
     blocks = std::min<int64_t>(blocks, (n + kWideThreads - 1) / kWideThreads);
     const bool stats = s->prof.level >= 2;
     const SceneRays src{(const WideNode*)s->wide.ptr, (const TriRec*)s->tris_wide.ptr, s->unculled, o, d, valid, perm,
-                        n, prim, t, b1, b2, occ};
+                        n, q.n_dev, prim, t, b1, b2, occ};
     auto kern = stats ? wide_walk_kernel<ANY, true, COOP, SceneRays> : wide_walk_kernel<ANY, false, COOP, SceneRays>;
     kern<<<(unsigned)blocks, kWideThreads, 0, st>>>(src, (int*)s->err.ptr, next,
                                                      stats ? (unsigned long long*)s->workc.ptr : nullptr);
@@ -466,15 +468,16 @@ int wide_launch(pbg_scene* s, const float4* o, const float4* d, const uint8_t* v
 }
 
 int wide_nearest(pbg_scene* s, bool coop, const float4* o, const float4* d, const uint8_t* valid,
-                 const int32_t* perm, int64_t n, int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st) {
-    return coop ? wide_launch<false, true>(s, o, d, valid, perm, n, prim, t, b1, b2, nullptr, st)
-                : wide_launch<false, false>(s, o, d, valid, perm, n, prim, t, b1, b2, nullptr, st);
+                 const int32_t* perm, int64_t n, QueueRef q, int32_t* prim, float* t, float* b1, float* b2,
+                 cudaStream_t st) {
+    return coop ? wide_launch<false, true>(s, o, d, valid, perm, n, q, prim, t, b1, b2, nullptr, st)
+                : wide_launch<false, false>(s, o, d, valid, perm, n, q, prim, t, b1, b2, nullptr, st);
 }
 
 int wide_occluded(pbg_scene* s, bool coop, const float4* o, const float4* d, const uint8_t* valid,
-                  const int32_t* perm, int64_t n, int32_t* occluders, uint8_t* occ, cudaStream_t st) {
-    return coop ? wide_launch<true, true>(s, o, d, valid, perm, n, occluders, nullptr, nullptr, nullptr, occ, st)
-                : wide_launch<true, false>(s, o, d, valid, perm, n, occluders, nullptr, nullptr, nullptr, occ, st);
+                  const int32_t* perm, int64_t n, QueueRef q, int32_t* occluders, uint8_t* occ, cudaStream_t st) {
+    return coop ? wide_launch<true, true>(s, o, d, valid, perm, n, q, occluders, nullptr, nullptr, nullptr, occ, st)
+                : wide_launch<true, false>(s, o, d, valid, perm, n, q, occluders, nullptr, nullptr, nullptr, occ, st);
 }
 
 }  // namespace pbg

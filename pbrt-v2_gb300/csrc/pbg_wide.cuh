@@ -427,13 +427,14 @@ struct SceneRays {
     const uint8_t* valid;
     const int32_t* perm;
     int64_t n;
+    const uint32_t* n_dev;  // the batch's length where the host does not know it
     int32_t* prim;
     float* t;
     float* b1;
     float* b2;
     uint8_t* occ;
 
-    __device__ __forceinline__ int64_t count() const { return n; }
+    __device__ __forceinline__ int64_t count() const { return n_dev ? (int64_t)*n_dev : n; }
     __device__ __forceinline__ bool fetch(int64_t slot, Lane& L, float4& o, float4& d) const {
         L.ray = perm ? (int64_t)perm[slot] : slot;
         if (valid != nullptr && valid[L.ray] == 0) return false;
