@@ -415,22 +415,36 @@ static int walk_counter(pbg_scene* s, const QueueRef& q, unsigned long long** ne
     return PBG_OK;
 }
 
-// The walk of a batch class (hint 1: incoherent).
-static int choose_walk(const pbg_scene* s, bool any, int hint) {
+// The walk of a batch class (hint 1: incoherent) of n rays.
+constexpr int64_t kPacketRays = 3 << 18;
+static int choose_walk(const pbg_scene* s, bool any, int hint, int64_t n) {
     if (s->params.walk != 0) return s->params.walk;
     const int tuned = s->tune.bvh_walk[any ? 1 : 0][hint == 1 ? 1 : 0];
     if (tuned != 0) return tuned;
-    // untuned: the walks the autotuner picked on both benchmark scenes' batch
-    // classes (camera rays 4; their shadow rays 5; bounce rays and their
-    // shadows 6), none of them more than 25 % off the class's best there
-    return hint == 1 ? 6 : (any ? 5 : 4);
+    // Untuned.  Bounce rays and their shadows: 6.  Coherent batches: packets
+    // (camera) and the lanes' own tests (shadows) pay once the batch fills the
+    // chip several times over; below that a packet's one dependent walk is the
+    // whole time.  Measured on terrains of 20,000 and 181,250 triangles and
+    // 1,024,000 triangles of spheres, us:
+    //   camera 500 rays      walk 4 217 / 288 / 370, 6  51 /  81 /  81, 2  60 / 90 / 90
+    //   camera 480,000       walk 4 154 / 274 / 425, 6 160 / 232 / 301
+    //   camera 1,048,576     walk 4 203 / 367 / 674, 6 271 / 439 / 672
+    //   shadow 500           walk 5  38 /  47 /  70, 6  33 /  41 /  65
+    //   shadow 480,000       walk 5  86 / 132 / 310, 6  90 / 130 / 268
+    //   shadow 1,048,576     walk 5 140 / 236 / 639, 6 150 / 242 / 550
+    //   shadow 4 to 8 M      walk 5 369 / 666 / 4337, 6 444 / 782 / 3868
+    // A scene that has traced only small camera batches has no eight-wide
+    // tree yet: walk 2 then, nearly as fast, instead of building one.
+    if (hint == 1) return 6;
+    if (any) return n < kPacketRays ? 6 : 5;
+    return n >= kPacketRays ? 4 : s->wide_state > 0 ? 6 : 2;
 }
 
 // Walk 3 sorts the batch and the learned ordering records it, both for a
 // length known to the host.
 bool bvh_queue_ok(const pbg_scene* s) {
     if (s->params.ray_sort > 0 || (s->learn && s->learn->enabled)) return false;
-    return choose_walk(s, false, 1) != 3 && choose_walk(s, true, 0) != 3 && choose_walk(s, true, 1) != 3;
+    return choose_walk(s, false, 1, 0) != 3 && choose_walk(s, true, 0, 0) != 3 && choose_walk(s, true, 1, 0) != 3;
 }
 
 // cluster_hint: a caller's cluster per ray (kNoCluster or any value outside
@@ -474,7 +488,7 @@ static int bvh_launch(pbg_scene* s, const float4* o, const float4* d, const uint
     // bounce batches are incoherent: the reference's bounce form of Intersect
     // is the one with a validity mask (rayhierarchy.cpp:602-813)
     const int hint = s->walk_hint >= 0 ? s->walk_hint : (!ANY && valid != nullptr ? 1 : 0);
-    int walk = choose_walk(s, ANY, hint);
+    int walk = choose_walk(s, ANY, hint, n);
     // Host-buffer calls run the packets in the caller's order: there the
     // batch arrives in parts whose copies overlap the traversal, and sorting
     // each part cost more than its packets gained (terrain frame end to end:
