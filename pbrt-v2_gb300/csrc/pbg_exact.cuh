@@ -47,6 +47,7 @@ struct __align__(16) TriRec {
 constexpr float kFilterC = 0x1p-19f;     // 32u
 constexpr float kFilterR = 0x1p-19f;     // threshold rounding margin
 constexpr float kFilterTiny = 0x1p-100f; // underflow guard
+constexpr float kFilterBig = 0x1p100f;   // products below 2^119: no overflow
 
 __device__ __forceinline__ float xcross(float a, float b, float c, float d) {
     // (a*b) - (c*d) evaluated in double, rounded once to float
@@ -111,7 +112,10 @@ __device__ __forceinline__ float flip_sign(float v, float s) {
 // best exact t so far, which the exact test accepts when equal).  nd = |d|_1.
 // Returns false only when pbg_exact() would return false for the same maxt.
 // stage2 (counting kernels only): incremented when the test goes past the
-// first barycentric check.
+// first barycentric check.  DEG: settle degenerate triangles here too (for
+// callers that test many of them; elsewhere the extra branch only costs:
+// 1,000,003 path bounces 1,042 -> 1,054 us).
+template <bool DEG = false>
 __device__ __forceinline__ bool pbg_filter(const TriRec& tr, float4 o, float4 d, float nd,
                                            float maxt, uint32_t* stage2 = nullptr) {
     const float e1x = tr.b.x, e1y = tr.b.y, e1z = tr.b.z;
@@ -128,12 +132,14 @@ __device__ __forceinline__ bool pbg_filter(const TriRec& tr, float4 o, float4 d,
     float ediv = fmaf(ck, ne1, kFilterTiny);  // bound on |div_f - div_ref|
     float e1b = fmaf(ck, nv, kFilterTiny);    // bound on |n1_f - n1_ref|
     float D = fabsf(div);
-    if (!(D > ediv))
-        // The divisor's sign (or zero) is uncertain, but it is at most D +
-        // ediv: a numerator above that makes |b1| > 1, rejected by either
-        // sign's check (a zero divisor is rejected anyway).  This settles
-        // nearly every test of a degenerate triangle, which every ray makes.
-        return !(fabsf(n1) - e1b > (D + ediv) * (1.f + 2.f * kFilterR));
+    if (!(D > ediv)) {  // sign of the divisor (or zero) uncertain
+        // ... but it is at most D + ediv: a numerator above that makes |b1| >
+        // 1, rejected by either sign's check (a zero divisor is rejected
+        // anyway).  Bounds this near the largest float mean that a product
+        // may overflow to a NaN, which pbrt's checks let pass.
+        return !DEG || !(fabsf(n1) - e1b > (D + ediv) * (1.f + 2.f * kFilterR)) ||
+               !(fmaxf(ck, fmaxf(ediv, e1b)) < kFilterBig);
+    }
     float a1 = flip_sign(n1, div);
     float top = fmaf(D, 1.f + kFilterR, ediv);
     if (a1 < -e1b || a1 > top + e1b) return false;

@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kNaiveThreads)
 
     auto test = [&](const TriRec& tr) {
         if (STATS) wc.filt++;
-        if (!pbg_filter(tr, o, d, nd, h.t, STATS ? &wc.filt2 : nullptr)) return;
+        if (!pbg_filter<true>(tr, o, d, nd, h.t, STATS ? &wc.filt2 : nullptr)) return;
         float tt, u1, u2;
         if (STATS) wc.exact++;
         if (!pbg_exact_rec(tr, o, d, h.t, &tt, &u1, &u2)) return;
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kNaiveThreads)
             if (lane < cnt) {
                 const TriRec own = rec[lane];
                 if (STATS) wc.filt++;
-                if (pbg_filter(own, oi, di, ni, mi, STATS ? &wc.filt2 : nullptr)) {
+                if (pbg_filter<true>(own, oi, di, ni, mi, STATS ? &wc.filt2 : nullptr)) {
                     if (STATS) wc.exact++;
                     hit = pbg_exact_rec(own, oi, di, mi, &tt, &b1, &b2);
                     if (STATS && hit) wc.hit++;

@@ -39,6 +39,47 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
     return d;
 }
 
+constexpr float kSlabWiden = 2.f * 3.f * 0x1p-24f / (1.f - 3.f * 0x1p-24f);
+
+// A ray for slab distances in one fused operation, t = plane * i + c with
+// c = -(o * i) rounded.  Against (plane - o) * i, whose rounding is relative
+// to t, the rounding of c adds u * |o * i| <= u * |t| + u * |plane * i|: the
+// first part keeps the three roundings that kSlabWiden covers, the second
+// moves the plane by u of its own magnitude, 2^-11 of the box's padding.
+// Where o * i overflows while o is finite, c is NaN and the axis is ignored
+// (fmax3 / fmin3 drop NaN), which keeps the box.
+struct RayFma {
+    float ix, iy, iz, cx, cy, cz;
+};
+
+__device__ __forceinline__ float slab_offset(float o, float i) {
+    const float c = -__fmul_rn(o, i);
+    return isinf(c) && !isinf(o) ? __int_as_float(0x7fffffff) : c;
+}
+
+__device__ __forceinline__ RayFma ray_fma(float4 o, float4 d) {
+    const float ix = safe_inv(d.x), iy = safe_inv(d.y), iz = safe_inv(d.z);
+    return RayFma{ix, iy, iz, slab_offset(o.x, ix), slab_offset(o.y, iy), slab_offset(o.z, iz)};
+}
+
+// Two fused multiply-adds in one instruction (sm_100 and later), each
+// rounded as fmaf.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+
+// Elements k, k + 1 (k even) of eight floats held as two float4.
+__device__ __forceinline__ float2 pair_of(const float4* v, int k) {
+    const float4 q = v[k >> 2];
+    return (k & 2) ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
+}
+
 __device__ __forceinline__ bool slab(const RayInv& r, float lx, float hx, float ly, float hy,
                                      float lz, float hz, float tmin, float tmax, float* tnear) {
     float tx0 = (lx - r.ox) * r.ix, tx1 = (hx - r.ox) * r.ix;
@@ -48,7 +89,7 @@ __device__ __forceinline__ bool slab(const RayInv& r, float lx, float hx, float 
     float tf = fmin3(fmaxf(tx0, tx1), fmaxf(ty0, ty1), fminf(fmaxf(tz0, tz1), tmax));
     *tnear = tn;
     // tf + |tf| * 2*gamma(3): each t carries at most two roundings
-    return tn <= fmaf(fabsf(tf), 2.f * 3.f * 0x1p-24f / (1.f - 3.f * 0x1p-24f), tf);
+    return tn <= fmaf(fabsf(tf), kSlabWiden, tf);
 }
 
 // The walk's stack.  PACK: one 8-byte entry (one local load per pop) when

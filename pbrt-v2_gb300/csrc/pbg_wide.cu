@@ -16,13 +16,12 @@
 //
 // Exactness.  The collapse keeps the binary tree's padded child boxes as
 // they are and only drops inner levels, so every triangle still sits inside
-// the boxes above it.  The slab test is the two-wide walk's, plane for plane
-// (t = (plane - o) * inv, far distance widened by 1 + 2 gamma(3)); the near
-// plane of each axis is picked by the sign of inv instead of a min/max of
-// the two planes' distances, which is the same value (the rounded
-// subtraction and product are monotone, and lo <= hi).  The leaf tests are
-// the same exact tests, so every walk returns the same prim, t, b1, b2 or
-// occlusion bit for bit.
+// the boxes above it.  The slab test takes each plane's distance in one fused
+// operation (RayFma in pbg_walk.cuh, two planes per instruction; its rounding
+// stays within the padding and the same widening, far distance times
+// 1 + 2 gamma(3)) and picks the near plane of each axis by the sign of inv.
+// The leaf tests are the same exact tests, so every walk returns the same
+// prim, t, b1, b2 or occlusion bit for bit.
 //
 // Built lazily on the first walk-5/6 batch of a scene: on the device from a
 // device-built tree (pbg_wide_build.cu), else on the host (collapse_wide).

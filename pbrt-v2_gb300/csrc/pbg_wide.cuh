@@ -82,12 +82,24 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     __shared__ CoopWarp coop[COOP ? kWideThreads / 32 : 1];
+    // eight hit bits in visiting order: bit k to bit k ^ order (a table: the
+    // three conditional swaps took 15 instructions a visit)
+    __shared__ uint8_t visit[8][256];
+    for (int i = threadIdx.x; i < 8 * 256; i += kWideThreads) {
+        uint32_t m = (uint32_t)i & 255u;
+        const uint32_t vo = (uint32_t)i >> 8;
+        if (vo & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
+        if (vo & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
+        if (vo & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
+        visit[vo][i & 255] = (uint8_t)m;
+    }
+    __syncthreads();
     int2 stack[kWideStack];  // (child base, hits | imask << 8 | distance bits)
     int sp = 0;
     typename Src::Lane L{};
     bool has = false, exhausted = false, ok = true, fin = false;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f), d = o;
-    RayInv ri{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    RayFma rf{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float nd = 0.f;
     WalkHit h{0.f, 0.f, 0.f, -1};
     uint32_t oct = 0;
@@ -131,9 +143,9 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                         finish();  // invalid: a miss, no walk
                     } else {
                         nd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
-                        ri = RayInv{o.x, o.y, o.z, safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)};
-                        oct = (__float_as_uint(ri.ix) >> 31) | (__float_as_uint(ri.iy) >> 31) << 1 |
-                              (__float_as_uint(ri.iz) >> 31) << 2;
+                        rf = ray_fma(o, d);
+                        oct = (__float_as_uint(rf.ix) >> 31) | (__float_as_uint(rf.iy) >> 31) << 1 |
+                              (__float_as_uint(rf.iz) >> 31) << 2;
                         h = WalkHit{d.w, 0.f, 0.f, -1};
                         sp = 0;
                         ok = true;
@@ -160,19 +172,27 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
             if (!__any_sync(full, searching)) break;
             // walk 6: the tests are dealt over the warp, so they need not
             // wait for the last searching lane: once four lanes hold two
-            // nodes' triangles the warp tests (path frame 1,319 -> 1,436
-            // Mrays/s; thresholds of 2, 3, 6, 8 lanes, or 8-20 lanes holding
-            // any: 1,356-1,435)
+            // nodes' triangles the warp tests (64 scenes 5.95 / 5.95 / 5.98 /
+            // 6.03 ms and path frame 18.9 / 18.9 / 19.0 / 19.2 ms for 3, 4, 6
+            // and 8 such lanes)
             if (COOP && __popc(__ballot_sync(full, has && tmask2 != 0)) >= 4) break;
+            // any-hit rays end at very different times: with 16 lanes idle
+            // the warp takes new rays (direct lighting 966 -> 933 us; for
+            // nearest hits 18.87 -> 19.12 ms, so not there)
+            if (ANY && __popc(__ballot_sync(full, !has && !exhausted)) >= 16) break;
             // a lane that holds triangles walks on for one more node's
             // triangles (two more when the warp deals its tests over its
             // lanes) while others search, so the tests below run with fuller
             // warps (walk 6 with two more: path bounces 1.66 -> 1.64 ms)
-            if (!has || (COOP ? tmask3 != 0 : tmask2 != 0) || rcnt != 0) continue;
-            if (ghits != 0 && gtn > h.t) ghits = 0;  // the whole group lies beyond the hit found
-            if (ghits == 0) {
-                bool got = false;
-                while (sp > 0) {
+            const bool act = has && !(COOP ? tmask3 != 0 : tmask2 != 0) && rcnt == 0;
+            // A lane out of children takes its next group here and visits it
+            // in the same step.  The barrier brings the warp back together:
+            // without it the compiler ran the visit once for the lanes that
+            // popped and once for the others (path frame 21.2 -> 23.3 ms; with
+            // it 19.6 -> 19.1 over popping in a step of its own).
+            if (act) {
+                if (ghits != 0 && gtn > h.t) ghits = 0;  // the whole group lies beyond the hit found
+                while (ghits == 0 && sp > 0) {
                     --sp;
                     const int2 e = stack[sp];
                     const float te = __uint_as_float((uint32_t)e.y & 0xffff0000u);
@@ -181,11 +201,13 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                         ghits = (uint32_t)e.y & 0xffu;
                         gimask = ((uint32_t)e.y >> 8) & 0xffu;
                         gtn = te;
-                        got = true;
-                        break;
                     }
                 }
-                if (!got && tmask == 0) finish();  // nothing left to walk or test
+            }
+            __syncwarp();
+            if (!act) continue;
+            if (ghits == 0) {
+                if (tmask == 0) finish();  // nothing left to walk or test
                 continue;
             }
             const int pos = __ffs(ghits) - 1;
@@ -193,43 +215,40 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
             const int cslot = pos ^ (int)visit_order_of<ANY>(oct);
             const int32_t child = gbase + __popc(gimask & ((1u << cslot) - 1u));
 
-            const float4* np = reinterpret_cast<const float4*>(src.nodes(L) + child);
-            const int4 r = __ldg(reinterpret_cast<const int4*>(np + 12));
-            // the near and far planes of the ray's octant, eight slots each
-            const int xo = (int)(oct & 1u) * 2, yo = 4 + (int)(oct & 2u), zo = 8 + (int)(oct & 4u) / 2;
-            const float4 nx0 = __ldg(np + xo), nx1 = __ldg(np + xo + 1);
-            const float4 fx0 = __ldg(np + (2 - xo)), fx1 = __ldg(np + (3 - xo));
-            const float4 ny0 = __ldg(np + yo), ny1 = __ldg(np + yo + 1);
-            const float4 fy0 = __ldg(np + (10 - yo)), fy1 = __ldg(np + (11 - yo));
-            const float4 nz0 = __ldg(np + zo), nz1 = __ldg(np + zo + 1);
-            const float4 fz0 = __ldg(np + (18 - zo)), fz1 = __ldg(np + (19 - zo));
-            const float nxs[8] = {nx0.x, nx0.y, nx0.z, nx0.w, nx1.x, nx1.y, nx1.z, nx1.w};
-            const float fxs[8] = {fx0.x, fx0.y, fx0.z, fx0.w, fx1.x, fx1.y, fx1.z, fx1.w};
-            const float nys[8] = {ny0.x, ny0.y, ny0.z, ny0.w, ny1.x, ny1.y, ny1.z, ny1.w};
-            const float fys[8] = {fy0.x, fy0.y, fy0.z, fy0.w, fy1.x, fy1.y, fy1.z, fy1.w};
-            const float nzs[8] = {nz0.x, nz0.y, nz0.z, nz0.w, nz1.x, nz1.y, nz1.z, nz1.w};
-            const float fzs[8] = {fz0.x, fz0.y, fz0.z, fz0.w, fz1.x, fz1.y, fz1.z, fz1.w};
-            const uint4 lt0 = __ldg(reinterpret_cast<const uint4*>(np + 13));
-            const uint4 lt1 = __ldg(reinterpret_cast<const uint4*>(np + 14));
+            // 32-bit offsets from the tree's base (under 2^24 nodes): fewer
+            // address instructions than a 64-bit pointer per plane
+            const char* nb = reinterpret_cast<const char*>(src.nodes(L));
+            const uint32_t at = (uint32_t)child * (uint32_t)sizeof(WideNode);
+            auto ld = [&](uint32_t word) { return __ldg(reinterpret_cast<const float4*>(nb + (at + word * 16u))); };
+            const int4 r = __ldg(reinterpret_cast<const int4*>(nb + (at + 192u)));
+            const uint32_t xo = (oct & 1u) * 2u, yo = 4u + (oct & 2u), zo = 8u + (oct & 4u) / 2u;
+            const float4 nx0 = ld(xo), nx1 = ld(xo + 1u), fx0 = ld(2u - xo), fx1 = ld(3u - xo);
+            const float4 ny0 = ld(yo), ny1 = ld(yo + 1u), fy0 = ld(10u - yo), fy1 = ld(11u - yo);
+            const float4 nz0 = ld(zo), nz1 = ld(zo + 1u), fz0 = ld(18u - zo), fz1 = ld(19u - zo);
+            const uint4 lt0 = __ldg(reinterpret_cast<const uint4*>(nb + (at + 208u)));
+            const uint4 lt1 = __ldg(reinterpret_cast<const uint4*>(nb + (at + 224u)));
             const uint32_t lts[8] = {lt0.x, lt0.y, lt0.z, lt0.w, lt1.x, lt1.y, lt1.z, lt1.w};
             const uint32_t imask = (uint32_t)r.x >> 24;
             uint32_t hits = 0, tm = 0;
             float ntn = INFINITY;  // nearest entry over the hit children: a bound for the group
+            const float2 ix2 = make_float2(rf.ix, rf.ix), iy2 = make_float2(rf.iy, rf.iy), iz2 = make_float2(rf.iz, rf.iz);
+            const float2 cx2 = make_float2(rf.cx, rf.cx), cy2 = make_float2(rf.cy, rf.cy), cz2 = make_float2(rf.cz, rf.cz);
+            const float4 nxs[2] = {nx0, nx1}, fxs[2] = {fx0, fx1}, nys[2] = {ny0, ny1}, fys[2] = {fy0, fy1},
+                         nzs[2] = {nz0, nz1}, fzs[2] = {fz0, fz1};
 #pragma unroll
-            for (int k = 0; k < kWideWidth; ++k) {
-                const float tnx = __fmul_rn(__fsub_rn(nxs[k], ri.ox), ri.ix);
-                const float tfx = __fmul_rn(__fsub_rn(fxs[k], ri.ox), ri.ix);
-                const float tny = __fmul_rn(__fsub_rn(nys[k], ri.oy), ri.iy);
-                const float tfy = __fmul_rn(__fsub_rn(fys[k], ri.oy), ri.iy);
-                const float tnz = __fmul_rn(__fsub_rn(nzs[k], ri.oz), ri.iz);
-                const float tfz = __fmul_rn(__fsub_rn(fzs[k], ri.oz), ri.iz);
-                const float tn = fmax3(tnx, tny, fmaxf(tnz, o.w));
-                const float tf = fmin3(tfx, tfy, fminf(tfz, h.t));
-                const bool hit = tn <= fmaf(fabsf(tf), 2.f * 3.f * 0x1p-24f / (1.f - 3.f * 0x1p-24f), tf);
-                if (hit) {
-                    hits |= 1u << k;
-                    tm |= lts[k];
-                    if (!ANY) ntn = fminf(ntn, tn);
+            for (int k = 0; k < kWideWidth; k += 2) {  // two boxes at a time
+                const float2 tnx = fma2(pair_of(nxs, k), ix2, cx2), tfx = fma2(pair_of(fxs, k), ix2, cx2);
+                const float2 tny = fma2(pair_of(nys, k), iy2, cy2), tfy = fma2(pair_of(fys, k), iy2, cy2);
+                const float2 tnz = fma2(pair_of(nzs, k), iz2, cz2), tfz = fma2(pair_of(fzs, k), iz2, cz2);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const float tn = fmax3(q ? tnx.y : tnx.x, q ? tny.y : tny.x, fmaxf(q ? tnz.y : tnz.x, o.w));
+                    const float tf = fmin3(q ? tfx.y : tfx.x, q ? tfy.y : tfy.x, fminf(q ? tfz.y : tfz.x, h.t));
+                    if (tn <= fmaf(fabsf(tf), kSlabWiden, tf)) {
+                        hits |= 1u << (k + q);
+                        tm |= lts[k + q];
+                        if (!ANY) ntn = fminf(ntn, tn);
+                    }
                 }
             }
             if (STATS) {
@@ -241,9 +260,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
             // hit inner children in visiting order: bit (slot ^ octant)
             uint32_t ih = hits & imask;
             const uint32_t vo = visit_order_of<ANY>(oct);
-            if (vo & 1u) ih = ((ih & 0x55u) << 1) | ((ih >> 1) & 0x55u);
-            if (vo & 2u) ih = ((ih & 0x33u) << 2) | ((ih >> 2) & 0x33u);
-            if (vo & 4u) ih = ((ih & 0x0fu) << 4) | ((ih >> 4) & 0x0fu);
+            ih = visit[vo][ih];
             if (ih) {
                 if (rest) {
                     if (sp < kWideStack) {
