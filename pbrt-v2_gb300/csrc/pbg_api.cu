@@ -258,23 +258,25 @@ static void prof_collect(pbg_scene* s) {
     }
 }
 
-// Stores the words, then (after a system-scope fence) the sequence number
-// in the last word: a host that sees the number sees the words.
 __global__ void publish_words_kernel(const int* __restrict__ src, int count, int* dst, int seq) {
-    if (threadIdx.x != 0) return;
-    volatile int* d = dst;
-    for (int k = 0; k < count; ++k) d[k] = src[k];
-    __threadfence_system();
-    d[kMailboxWords - 1] = seq;
+    if (threadIdx.x == 0) publish_words(src, count, dst, seq);
 }
 
-int publish_device_words(pbg_scene* s, const int* dev, int count, int* seq_out, cudaStream_t st) {
-    if (count > kMailboxWords - 1 || !s->mbox_dev) return PBG_ERR_INVALID_ARGUMENT;
-    const int seq = (int)++s->mbox_seq;  // compared as bits; wraps harmlessly
-    publish_words_kernel<<<1, 32, 0, st>>>(dev, count, s->mbox_dev, seq);
+int next_publication(pbg_scene* s, int** dst, int* seq) {
+    if (!s->mbox_dev) return PBG_ERR_INVALID_ARGUMENT;
+    *dst = s->mbox_dev;
+    *seq = (int)++s->mbox_seq;  // compared as bits; wraps harmlessly
+    return PBG_OK;
+}
+
+int publish_device_words(pbg_scene* s, const int* dev, int count, int* seq, cudaStream_t st) {
+    if (count > kMailboxWords - 1) return PBG_ERR_INVALID_ARGUMENT;
+    int* dst = nullptr;
+    const int rc = next_publication(s, &dst, seq);
+    if (rc) return rc;
+    publish_words_kernel<<<1, 32, 0, st>>>(dev, count, dst, *seq);
     s->counters.kernel_launches++;
     PBG_CUDA(cudaGetLastError());
-    *seq_out = seq;
     return PBG_OK;
 }
 

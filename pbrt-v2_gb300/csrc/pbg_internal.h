@@ -221,9 +221,21 @@ void render_free(pbg_scene* s);
 constexpr int kMailboxWords = 16;
 int read_device_words(pbg_scene* s, const int* dev, int count, int* out, cudaStream_t st);
 // The two halves of read_device_words: work enqueued between them runs while
-// the host waits for the words.
+// the host waits for the words.  A kernel may publish by itself instead
+// (publish_words with the mailbox and number of next_publication).
 int publish_device_words(pbg_scene* s, const int* dev, int count, int* seq, cudaStream_t st);
+int next_publication(pbg_scene* s, int** dst, int* seq);
 int wait_device_words(pbg_scene* s, int seq, int count, int* out, cudaStream_t st);
+#ifdef __CUDACC__
+// Stores the words, then (after a system-scope fence) the sequence number
+// in the last word: a host that sees the number sees the words.
+__device__ __forceinline__ void publish_words(const int* src, int count, int* dst, int seq) {
+    volatile int* d = dst;
+    for (int k = 0; k < count; ++k) d[k] = src[k];
+    __threadfence_system();
+    d[kMailboxWords - 1] = seq;
+}
+#endif
 
 // Stage timing around one launch (no-ops unless profiling is on); stages:
 // 0 ray sort, 1 hierarchy build, 2 traversal, 3 finalize / other.

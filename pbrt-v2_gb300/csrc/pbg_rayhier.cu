@@ -74,16 +74,42 @@ __device__ __forceinline__ float round_up_rel(float x) { return fmaf(fabsf(x), 0
 
 // ---------------------------------------------------------------- build
 
+// A batch of at most this many rays has launches and few long pairs to wait
+// for: its leaf build zeroes the traversal's words, its finalize kernel
+// publishes the status, and its split tests take a leaf per warp; larger
+// batches use memsets, a kernel of its own and a pair per warp.  Frames of
+// 130,000 / 350,000 rays x 2 samples / 1024 x 1024 x 4 samples: 498 / 1,766 /
+// 4,006 us in the first form, 561 / 1,826 / 3,686 in the second.
+constexpr int64_t kFewRays = 1 << 20;
+
+// Words of device memory that a batch starts from zero (its keys or
+// occlusion bits, counters, bounds).
+constexpr int kZeroRanges = 6;
+struct ZeroWords {
+    uint32_t* p[kZeroRanges] = {};
+    int64_t n[kZeroRanges] = {};
+    int count = 0;
+    void add(void* ptr, size_t bytes) {  // a multiple of 4 bytes
+        p[count] = (uint32_t*)ptr;
+        n[count++] = (int64_t)(bytes / 4);
+    }
+};
+
 // One warp per leaf of 32 sorted rays; the warp also gathers its rays into
 // sorted order (so, sd) for the leaf tests.
 // keep_o: the batch leaves from the same origins (bit for bit, mint
 // included) in the same order as the previous one, whose sorted origins and
 // leaf spheres are still in so / leaves: only the directions are gathered
 // and only the cones rebuilt.
+template <bool ZERO>
 __global__ void leaf_build_kernel(const float4* __restrict__ ro, const float4* __restrict__ rd,
                                   const int32_t* __restrict__ perm, float4* __restrict__ so,
                                   float4* __restrict__ sd, const uint32_t* __restrict__ skeys, int64_t n,
-                                  int64_t nleaf, RayNode* __restrict__ leaves, bool keep_o) {
+                                  int64_t nleaf, RayNode* __restrict__ leaves, bool keep_o, const ZeroWords zero) {
+    for (int k = 0; ZERO && k < zero.count; ++k)
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < zero.n[k];
+             i += (int64_t)gridDim.x * blockDim.x)
+            zero.p[k][i] = 0u;
     const int64_t leaf = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (leaf >= nleaf) return;
@@ -419,7 +445,11 @@ __device__ __forceinline__ void lower_reach(uint32_t* b, float x) {
     atomicMax(b, 0x7f800000u - __float_as_uint(x));
 }
 
-template <bool ANY, bool STATS>
+// SMALL (batches of at most kFewRays rays): a warp takes one leaf of a pair
+// and tests the members against the parent again, since with few pairs to a
+// warp the longest one is the kernel's time (a frame of 19,159 rays 228 us ->
+// 198).
+template <bool ANY, bool STATS, bool SMALL>
 __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBlocks)
     rh_split_test_kernel(const float4* __restrict__ spheres, const TriRec* __restrict__ tris, int32_t t0,
                          int32_t t1, const RayNode* __restrict__ level1, const RayNode* __restrict__ leaves,
@@ -437,8 +467,9 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     WorkCount c_;
-    for (int64_t p = warp; p < nin; p += nwarps) {
-        const Pair pr = in[p];
+    const int64_t ntask = SMALL ? (int64_t)nin * kFan : nin;
+    for (int64_t task = warp; task < ntask; task += nwarps) {
+        const Pair pr = in[SMALL ? task / kFan : task];
         const int64_t t = (int64_t)pr.tri * kClusterTris + lane;
         bool pass = false;
         float4 sph = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -465,7 +496,7 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
         const int64_t first = (int64_t)pr.node * kFan;
         float parent_new = 0.f;  // max of the leaves' bounds after this pair
 #pragma unroll 1
-        for (int c = 0; c < kFan; ++c) {
+        for (int c = SMALL ? (int)(task % kFan) : 0, c1 = SMALL ? c + 1 : kFan; c < c1; ++c) {
             const int64_t leaf = first + c;
             if (leaf >= nleaf) break;
             RayNode nd = leaves[leaf];
@@ -540,7 +571,7 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
                 parent_new = fmaxf(parent_new, fminf(b, nd.c.y));
             }
         }
-        if (!ANY && lane == 0 && parent_new < parent_now) lower_reach(parent_reach + pr.node, parent_new);
+        if (!ANY && !SMALL && lane == 0 && parent_new < parent_now) lower_reach(parent_reach + pr.node, parent_new);
     }
     if (STATS) c_.flush(wc);
 }
@@ -741,12 +772,24 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
     if (STATS) c_.flush(wc);
 }
 
+// The batch's status words to the host, from the finalize kernel's first
+// thread: the kernel starts behind the leaf tests that set them.
+struct Publication {
+    const int* src = nullptr;
+    int* dst = nullptr;
+    int count = 0, seq = 0;
+};
+__device__ __forceinline__ void publish(const Publication& pub) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && pub.count > 0) publish_words(pub.src, pub.count, pub.dst, pub.seq);
+}
+
 // Sorted-order results back to the caller's order.
 __global__ void rh_finalize_nearest(const TriRec* __restrict__ tris, const int32_t* __restrict__ pos,
                                     const float4* __restrict__ so, const float4* __restrict__ sd,
                                     const int32_t* __restrict__ perm,
                                     const unsigned long long* __restrict__ keys, int64_t n,
-                                    int32_t* prim, float* t, float* b1, float* b2) {
+                                    int32_t* prim, float* t, float* b1, float* b2, const Publication pub) {
+    publish(pub);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int32_t ray = perm[i];
@@ -769,7 +812,8 @@ __global__ void rh_finalize_nearest(const TriRec* __restrict__ tris, const int32
 
 __global__ void rh_finalize_occluded(const int32_t* __restrict__ perm,
                                      const uint32_t* __restrict__ leafmask, int64_t n,
-                                     uint8_t* occ) {
+                                     uint8_t* occ, const Publication pub) {
+    publish(pub);
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     occ[perm[i]] = (leafmask[i / kLeafRays] >> (i % kLeafRays)) & 1u;
@@ -800,8 +844,11 @@ static Descent descent_levels(const pbg_scene* s, const Levels& lv, bool any) {
     return d;
 }
 
+static int rh_workspace(pbg_scene* s, const Levels& lv, bool any, ZeroWords* zero);
+
+// zero: what the caller needs zeroed, to which the traversal's words are added.
 static int rh_build(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
-                    const int32_t** perm, float4** so, float4** sd, Levels* lv, int order,
+                    const int32_t** perm, float4** so, float4** sd, Levels* lv, int order, ZeroWords* zero,
                     cudaStream_t st) {
     Work& w = s->work;
     const uint32_t* skeys = nullptr;
@@ -833,9 +880,12 @@ static int rh_build(pbg_scene* s, const float4* o, const float4* d, const uint8_
     // its order was reused and neither buffer moved
     const bool keep_o = order == kOrderOrigin && w.origin_reused && had_origins &&
                         before[0] == w.ray_o2.ptr && before[1] == w.nodes.ptr;
+    if (s->ntri > 0 && (rc = rh_workspace(s, *lv, order == kOrderOrigin, zero))) return rc;
+    const bool few = n <= kFewRays;
+    for (int k = 0; !few && k < zero->count; ++k) PBG_CUDA(cudaMemsetAsync(zero->p[k], 0, (size_t)zero->n[k] * 4, st));
     prof_begin(s, st);
-    leaf_build_kernel<<<(unsigned)((nleaf * 32 + 255) / 256), 256, 0, st>>>(o, d, *perm, *so, *sd, skeys,
-                                                                            n, nleaf, nodes, keep_o);
+    (few ? leaf_build_kernel<true> : leaf_build_kernel<false>)<<<(unsigned)((nleaf * 32 + 255) / 256), 256, 0, st>>>(
+        o, d, *perm, *so, *sd, skeys, n, nleaf, nodes, keep_o, *zero);
     prof_end(s, st, kStageBuild, 1);
     // the levels above are never read (any-hit batches are the origin-ordered ones)
     const int built = descent_levels(s, *lv, order == kOrderOrigin).seed;
@@ -863,20 +913,44 @@ static uint32_t queue_capacity(const pbg_scene* s) {
     return q > 0 ? std::max<uint32_t>((uint32_t)q, kQueueCapMin) : kQueueCap;
 }
 
-template <bool ANY>
-static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const float4* sd,
-                       unsigned long long* keys, uint32_t* mask, cudaStream_t st, int* moved,
-                       const std::function<int()>& tail) {
+// Live reach bounds of a nearest-hit batch (words of Work::reach): leaves,
+// their parents, then the pair order's buckets.
+static bool rh_has_reach(const Levels& lv, bool any) { return !any && lv.nlev > 1; }
+static size_t rh_reach_words(const Levels& lv) { return ((size_t)(lv.cnt[0] + lv.cnt[1]) + 3) / 4 * 4; }  // buckets aligned for the scan
+
+// The traversal's buffers, and the words of them that start from zero.
+static int rh_workspace(pbg_scene* s, const Levels& lv, bool any, ZeroWords* zero) {
     Work& w = s->work;
     int rc;
-    const int64_t nleaf = lv.cnt[0];
     const uint32_t cap = queue_capacity(s);
     if ((rc = ensure(w.queue_a, (size_t)cap * sizeof(Pair))) ||
         (rc = ensure(w.queue_b, (size_t)cap * sizeof(Pair))) ||
         (rc = ensure(w.pair_rank, (size_t)cap * sizeof(uint32_t))) ||
-        (rc = ensure(w.leafcnt, (size_t)nleaf * sizeof(uint32_t))) ||
+        (rc = ensure(w.leafcnt, (size_t)lv.cnt[0] * sizeof(uint32_t))) ||
         (rc = ensure(w.qcount, 64 * sizeof(uint32_t))))
         return rc;
+    zero->add(w.qcount.ptr, 64 * sizeof(uint32_t));
+    zero->add((int*)s->err.ptr + kStatusOverflow, sizeof(int));
+    const int split = descent_levels(s, lv, any).split;
+    if (!(split == 1 && lv.nlev - 1 > split))  // the leaf-pair counting sort runs
+        zero->add(w.leafcnt.ptr, (size_t)lv.cnt[0] * sizeof(uint32_t));
+    if (rh_has_reach(lv, any)) {
+        const size_t bytes = (rh_reach_words(lv) + kOrderBuckets) * sizeof(uint32_t);
+        if ((rc = ensure(w.reach, bytes))) return rc;
+        zero->add(w.reach.ptr, bytes);
+    }
+    return PBG_OK;
+}
+
+// rh_build has run with the words of rh_workspace zeroed.
+template <bool ANY>
+static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const float4* sd,
+                       unsigned long long* keys, uint32_t* mask, cudaStream_t st, int* moved,
+                       const std::function<int(const Publication&)>& finalize) {
+    Work& w = s->work;
+    int rc;
+    const int64_t nleaf = lv.cnt[0];
+    const uint32_t cap = queue_capacity(s);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
     // grid-stride kernels: 32 CTAs per SM measured best of 4, 8, 16, 32 on
@@ -896,23 +970,21 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
     const float4* tsph = (const float4*)s->spheres.ptr;
     const float4* csph = (const float4*)s->clusters.ptr;
     uint32_t *leaf_reach = nullptr, *parent_reach = nullptr, *order_hist = nullptr;
-    if (!ANY && lv.nlev > 1) {  // live reach bounds, +inf to start (zeroed)
-        const size_t nb = (size_t)(lv.cnt[0] + lv.cnt[1]);
-        if ((rc = ensure(w.reach, (nb + kOrderBuckets) * sizeof(uint32_t)))) return rc;
+    if (rh_has_reach(lv, ANY)) {  // live reach bounds, +inf to start (zeroed)
         leaf_reach = (uint32_t*)w.reach.ptr;
         parent_reach = leaf_reach + lv.cnt[0];
-        order_hist = parent_reach + lv.cnt[1];
-        PBG_CUDA(cudaMemsetAsync(leaf_reach, 0, nb * sizeof(uint32_t), st));
+        order_hist = leaf_reach + rh_reach_words(lv);
     }
     for (int attempt = 0; attempt < 8; ++attempt) {
-        PBG_CUDA(cudaMemsetAsync(status + kStatusOverflow, 0, sizeof(int), st));
+        if (attempt > 0) PBG_CUDA(cudaMemsetAsync(status + kStatusOverflow, 0, sizeof(int), st));
         // group boundaries on cluster boundaries
         const int64_t per = ((s->ntri + groups - 1) / groups + kClusterTris - 1) / kClusterTris * kClusterTris;
         for (int g = 0; g < groups; ++g) {
             const int32_t t0 = (int32_t)std::min<int64_t>(s->ntri, g * per),
                           t1 = (int32_t)std::min<int64_t>(s->ntri, (g + 1) * per);
             if (t0 >= t1) break;
-            PBG_CUDA(cudaMemsetAsync(counts, 0, 64 * sizeof(uint32_t), st));
+            const bool fresh = attempt == 0 && g == 0;  // rh_build zeroed the counters
+            if (!fresh) PBG_CUDA(cudaMemsetAsync(counts, 0, 64 * sizeof(uint32_t), st));
             Pair* qa = (Pair*)w.queue_a.ptr;
             Pair* qb = (Pair*)w.queue_b.ptr;
             prof_begin(s, st);
@@ -938,14 +1010,14 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
                     nullptr);
             uint32_t* leafcnt = (uint32_t*)w.leafcnt.ptr;
             uint32_t* rank = (uint32_t*)w.pair_rank.ptr;
-            if (!(cl && split == 1))  // the leaf-pair counting sort runs
+            if (!fresh && !(cl && split == 1))  // the leaf-pair counting sort runs
                 PBG_CUDA(cudaMemsetAsync(leafcnt, 0, (size_t)nleaf * sizeof(uint32_t), st));
             bool fused = false;
             for (int l = ls; l >= 0; --l) {
                 if (cl && l == 1 && split == 1) {  // clusters straight into the leaf tests
                     unsigned tgrid = grid * 2;
                     if (order_hist) {  // nearest: front-to-back pairs, taken in order
-                        PBG_CUDA(cudaMemsetAsync(order_hist, 0, kOrderBuckets * sizeof(uint32_t), st));
+                        if (!fresh) PBG_CUDA(cudaMemsetAsync(order_hist, 0, kOrderBuckets * sizeof(uint32_t), st));
                         rh_order_count_kernel<<<grid, 256, 0, st>>>(csph, nodes + lv.off[1], qa, cnt_of[1],
                                                                     cap, order_hist, status);
                         if ((rc = scan_counts(s, order_hist, kOrderBuckets, st))) return rc;
@@ -958,16 +1030,12 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
                         tgrid = (unsigned)(sms * kNearestMinBlocks);  // resident CTAs only
                         nl += 2;
                     }
-                    if (stats)
-                        rh_split_test_kernel<ANY, true><<<tgrid, 256, 0, st>>>(
-                            tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1], nodes + lv.off[0],
-                            lv.cnt[0], qa, cnt_of[1], cap, so, sd, keys, mask, leaf_reach,
-                            parent_reach, status, wc);
-                    else
-                        rh_split_test_kernel<ANY, false><<<tgrid, 256, 0, st>>>(
-                            tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1], nodes + lv.off[0],
-                            lv.cnt[0], qa, cnt_of[1], cap, so, sd, keys, mask, leaf_reach,
-                            parent_reach, status, nullptr);
+                    const auto kernel = stats ? rh_split_test_kernel<ANY, true, false>
+                                        : nleaf * kLeafRays <= kFewRays ? rh_split_test_kernel<ANY, false, true>
+                                                                        : rh_split_test_kernel<ANY, false, false>;
+                    kernel<<<tgrid, 256, 0, st>>>(tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1],
+                                                  nodes + lv.off[0], lv.cnt[0], qa, cnt_of[1], cap, so, sd, keys, mask,
+                                                  leaf_reach, parent_reach, status, stats ? wc : nullptr);
                     fused = true;
                     ++nl;
                     break;
@@ -1024,14 +1092,22 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
         // One status read per call: a dropped pair would lose hits.  With
         // *moved, the word after it too: the batch's origins differ from
         // the kept order it was traced in, and the caller traces it again.
-        // The caller's tail (the finalize kernel) is enqueued behind the
-        // publication, so the GPU runs it while the host waits; an attempt
-        // that is rerun enqueues it again.
-        int seq = 0;
-        if ((rc = publish_device_words(s, status + kStatusOverflow, moved ? 2 : 1, &seq, st))) return rc;
-        if ((rc = tail())) return rc;
+        // The finalize kernel runs while the host waits; an attempt that is
+        // rerun runs it again.  A small batch's finalize publishes the words
+        // itself (a launch less); among a large one's stores the words would
+        // reach the host some 15 us later than from a kernel before it.
+        Publication pub;
+        const int words = moved ? 2 : 1;
+        if (nleaf * kLeafRays <= kFewRays) {
+            pub.count = words;
+            pub.src = status + kStatusOverflow;
+            if ((rc = next_publication(s, &pub.dst, &pub.seq))) return rc;
+        } else if ((rc = publish_device_words(s, status + kStatusOverflow, words, &pub.seq, st))) {
+            return rc;
+        }
+        if ((rc = finalize(pub))) return rc;
         int h[2] = {0, 0};
-        if ((rc = wait_device_words(s, seq, moved ? 2 : 1, h, st))) return rc;
+        if ((rc = wait_device_words(s, pub.seq, words, h, st))) return rc;
         if (moved && h[1] != 0) {
             *moved = 1;
             return PBG_OK;
@@ -1056,23 +1132,24 @@ int rh_nearest(pbg_scene* s, const float4* o, const float4* d, const uint8_t* va
     const int32_t* perm;
     float4 *so, *sd;
     Levels lv;
-    int rc = rh_build(s, o, d, valid, n, &perm, &so, &sd, &lv, kOrderDefault, st);
-    if (rc) return rc;
     Work& w = s->work;
+    int rc;
     if ((rc = ensure(w.keys, (size_t)n * 8))) return rc;
     unsigned long long* keys = (unsigned long long*)w.keys.ptr;
-    PBG_CUDA(cudaMemsetAsync(keys, 0, (size_t)n * 8, st));
-    const std::function<int()> finalize = [&]() -> int {
+    ZeroWords zero;
+    zero.add(keys, (size_t)n * 8);
+    if ((rc = rh_build(s, o, d, valid, n, &perm, &so, &sd, &lv, kOrderDefault, &zero, st))) return rc;
+    const std::function<int(const Publication&)> finalize = [&](const Publication& pub) -> int {
         prof_begin(s, st);
         rh_finalize_nearest<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
             (const TriRec*)s->tris.ptr, (const int32_t*)s->tri_pos.ptr, so, sd, perm, keys, n, prim, t, b1,
-            b2);
+            b2, pub);
         prof_end(s, st, kStageOther, 1);
         PBG_CUDA(cudaGetLastError());
         return PBG_OK;
     };
     if (s->ntri > 0) return rh_traverse<false>(s, lv, so, sd, keys, nullptr, st, nullptr, finalize);
-    return finalize();
+    return finalize(Publication());
 }
 
 int rh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
@@ -1085,17 +1162,18 @@ int rh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* v
         const int32_t* perm;
         float4 *so, *sd;
         Levels lv;
-        int rc = rh_build(s, o, d, valid, n, &perm, &so, &sd, &lv, kOrderOrigin, st);
-        if (rc) return rc;
         Work& w = s->work;
-        const bool speculative = w.origin_speculative;
-        const int64_t nleaf = lv.cnt[0];
-        if ((rc = ensure(w.leafmask, (size_t)nleaf * 4))) return rc;
+        const size_t mask_bytes = (size_t)((n + kLeafRays - 1) / kLeafRays) * 4;
+        int rc;
+        if ((rc = ensure(w.leafmask, mask_bytes))) return rc;
         uint32_t* mask = (uint32_t*)w.leafmask.ptr;
-        PBG_CUDA(cudaMemsetAsync(mask, 0, (size_t)nleaf * 4, st));
-        const std::function<int()> finalize = [&]() -> int {
+        ZeroWords zero;
+        zero.add(mask, mask_bytes);
+        if ((rc = rh_build(s, o, d, valid, n, &perm, &so, &sd, &lv, kOrderOrigin, &zero, st))) return rc;
+        const bool speculative = w.origin_speculative;
+        const std::function<int(const Publication&)> finalize = [&](const Publication& pub) -> int {
             prof_begin(s, st);
-            rh_finalize_occluded<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(perm, mask, n, occ);
+            rh_finalize_occluded<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(perm, mask, n, occ, pub);
             prof_end(s, st, kStageOther, 1);
             PBG_CUDA(cudaGetLastError());
             return PBG_OK;
@@ -1107,7 +1185,7 @@ int rh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* v
             rc = rh_traverse<true>(s, lv, so, sd, nullptr, mask, st, speculative ? &moved : nullptr, finalize);
             if (rc) return rc;
         } else {
-            if ((rc = finalize())) return rc;
+            if ((rc = finalize(Publication()))) return rc;
             if (speculative &&
                 (rc = read_device_words(s, (const int*)s->err.ptr + kStatusOriginMoved, 1, &moved, st)))
                 return rc;
