@@ -61,7 +61,7 @@ constexpr int kMaxLevels = 16;
 struct __align__(16) RayNode {
     float4 a;  // origin sphere: centre.xyz, radius
     float4 b;  // cone axis.xyz, cos(half-angle)
-    float4 c;  // sin(half-angle), reach = max maxt*|d|, count (int bits), unused
+    float4 c;  // sin(half-angle), reach = max maxt*|d|, count (int bits), spread (beam_spread)
 };
 
 struct Levels {
@@ -74,13 +74,22 @@ __device__ __forceinline__ float round_up_rel(float x) { return fmaf(fabsf(x), 0
 
 // ---------------------------------------------------------------- build
 
+// An upper bound on |u - axis| over the unit directions u of a cone with
+// cosine c (already lowered by its rounding), or +inf where a ray's length is
+// extreme (beam_misses' bounds then do not hold).
+constexpr float kPlainDir = 0x1p30f;
+__device__ __forceinline__ float beam_spread(float c, bool plain) {
+    return plain ? sqrtf(2.f * (1.f - c)) * (1.f + 0x1p-16f) : INFINITY;
+}
+
 // A batch of at most this many rays has launches and few long pairs to wait
 // for: its leaf build zeroes the traversal's words, its finalize kernel
-// publishes the status, and its split tests take a leaf per warp; larger
-// batches use memsets, a kernel of its own and a pair per warp.  Frames of
-// 130,000 / 350,000 rays x 2 samples / 1024 x 1024 x 4 samples: 498 / 1,766 /
-// 4,006 us in the first form, 561 / 1,826 / 3,686 in the second.
-constexpr int64_t kFewRays = 1 << 20;
+// publishes the status, its split tests take a leaf per warp and its other
+// kernels fewer CTAs; larger batches use memsets, a kernel of its own and a
+// pair per warp.  Frames of 131,400 / 256,000 / 700,000 rays: 452 / 618 /
+// 1,664 us in the first form, 469 / 624 / 1,439 in the second.
+constexpr int64_t kFewRays = 1 << 19;
+constexpr int kFewGrid = 12;  // CTAs per SM of their level kernels (of 4, 12, 32: 175, 172, 177 us at 19,159 rays)
 
 // Words of device memory that a batch starts from zero (its keys or
 // occlusion bits, counters, bounds).
@@ -94,6 +103,19 @@ struct ZeroWords {
         n[count++] = (int64_t)(bytes / 4);
     }
 };
+
+// The least / greatest of the warp's values, NaN ignored as by fminf / fmaxf
+// (one instruction, sm_100 and later, for ten of a shuffle tree).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
 
 // One warp per leaf of 32 sorted rays; the warp also gathers its rays into
 // sorted order (so, sd) for the leaf tests.
@@ -129,6 +151,11 @@ __global__ void leaf_build_kernel(const float4* __restrict__ ro, const float4* _
     const int count = __popc(__ballot_sync(full, ok));
     float lo[3] = {ok ? o.x : INFINITY, ok ? o.y : INFINITY, ok ? o.z : INFINITY};
     float hi[3] = {ok ? o.x : -INFINITY, ok ? o.y : -INFINITY, ok ? o.z : -INFINITY};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = warp_min(lo[a]);
+        hi[a] = warp_max(hi[a]);
+    }
     const float len = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
     const float il = len > 0.f ? 1.f / len : 0.f;
     float nx = d.x * il, ny = d.y * il, nz = d.z * il;
@@ -137,15 +164,11 @@ __global__ void leaf_build_kernel(const float4* __restrict__ ro, const float4* _
     if (ok && !(reach == reach)) reach = INFINITY;  // 0 * inf
 #pragma unroll
     for (int off = 16; off; off >>= 1) {
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(full, lo[a], off));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(full, hi[a], off));
-        }
         sx += __shfl_xor_sync(full, sx, off);
         sy += __shfl_xor_sync(full, sy, off);
         sz += __shfl_xor_sync(full, sz, off);
-        reach = fmaxf(reach, __shfl_xor_sync(full, reach, off));
     }
+    reach = warp_max(reach);
     const float cx = 0.5f * (lo[0] + hi[0]), cy = 0.5f * (lo[1] + hi[1]), cz = 0.5f * (lo[2] + hi[2]);
     float dist = ok ? sqrtf((o.x - cx) * (o.x - cx) + (o.y - cy) * (o.y - cy) + (o.z - cz) * (o.z - cz)) : 0.f;
     const float sl = sqrtf(sx * sx + sy * sy + sz * sz);
@@ -158,11 +181,9 @@ __global__ void leaf_build_kernel(const float4* __restrict__ ro, const float4* _
     }
     float cosv = ok ? (axis_ok ? ax * nx + ay * ny + az * nz : -1.f) : 2.f;
     if (ok && !(len > 0.f && isfinite(len))) cosv = -1.f;
-#pragma unroll
-    for (int off = 16; off; off >>= 1) {
-        dist = fmaxf(dist, __shfl_xor_sync(full, dist, off));
-        cosv = fminf(cosv, __shfl_xor_sync(full, cosv, off));
-    }
+    const bool plain = __all_sync(full, !ok || (len >= 1.f / kPlainDir && len <= kPlainDir));
+    dist = warp_max(dist);
+    cosv = warp_min(cosv);
     if (lane == 0) {
         RayNode nd;
         if (count == 0) {
@@ -177,7 +198,7 @@ __global__ void leaf_build_kernel(const float4* __restrict__ ro, const float4* _
             const float s = fminf(sqrtf(fmaxf(0.f, 1.f - c * c)) + 0x1p-18f, 1.f);
             nd.a = keep_o ? leaves[leaf].a : make_float4(cx, cy, cz, ro_);
             nd.b = make_float4(ax, ay, az, c);
-            nd.c = make_float4(s, reach, __int_as_float(count), 0.f);
+            nd.c = make_float4(s, reach, __int_as_float(count), beam_spread(c, plain));
         }
         leaves[leaf] = nd;
     }
@@ -291,6 +312,48 @@ __device__ __forceinline__ bool node_hits_sphere(const RayNode& nd, float4 sph) 
     if (cth * dist <= -q) return true;  // cone half-angle + sphere angle >= pi
     const float dotv = vx * nd.b.x + vy * nd.b.y + vz * nd.b.z;
     return dotv >= cth * q - sth * R - 0x1p-16f * dist_hi;
+}
+
+// Whether every ray of a leaf certainly misses the triangle: pbrt's test,
+// s1 = d x e2, div = s1.e1, b1 = (v.s1) / div, b2 = (d.(v x e1)) / div with
+// v = o - p1, over all origins within r of the leaf's centre and unit
+// directions u within the spread of its axis a.  With w = centre - p1, for
+// every ray
+//   div / |d|          = u.(e2 x e1)  is within spread |e2 x e1| of a.(e2 x e1),
+//   (b1 div) / |d|     = u.(e2 x v)   within spread |e2 x w| + |e2| r of a.(e2 x w),
+//   (b2 div) / |d|     = u.(v x e1)   within spread |w x e1| + |e1| r of a.(w x e1),
+//   ((b1 + b2 - 1) div) / |d|, the sum of the last two less the first,
+//                      = u.((e2 - e1) x (v - e1)), its bound likewise.
+// So the triangle is missed where the divisor's sign is certain and b1 < 0,
+// b2 < 0 or b1 + b2 > 1 for all of them.  2^-17 of the lengths covers pbrt's
+// rounding of each product (9.1 u with u = 2^-24, see pbg_exact.cuh), the
+// rounding here and that of b1, b2 and their sum; edges, distances and
+// directions of extreme size, where products may overflow or underflow, are
+// never missed, and a NaN anywhere keeps the triangle.
+__device__ __forceinline__ float rough_len(float x, float y, float z) {
+    const float l2 = x * x + y * y + z * z;
+    return l2 * rsqrtf(l2);  // within 2^-20, inside the spread's own margin
+}
+__device__ __forceinline__ bool beam_misses(const RayNode& nd, const TriRec& tr) {
+    constexpr float kTol = 0x1p-17f, kBig = 0x1p29f;
+    const float e1x = tr.b.x, e1y = tr.b.y, e1z = tr.b.z, e2x = tr.c.x, e2y = tr.c.y, e2z = tr.c.z;
+    const float ne1 = tr.a.w, ne2 = tr.b.w, r = nd.a.w, spread = nd.c.w;
+    const float wx = nd.a.x - tr.a.x, wy = nd.a.y - tr.a.y, wz = nd.a.z - tr.a.z;
+    const float nw = fabsf(wx) + fabsf(wy) + fabsf(wz) + r;
+    const float mx = fmaf(e2y, e1z, -(e2z * e1y)), my = fmaf(e2z, e1x, -(e2x * e1z)), mz = fmaf(e2x, e1y, -(e2y * e1x));
+    const float q1x = fmaf(e2y, wz, -(e2z * wy)), q1y = fmaf(e2z, wx, -(e2x * wz)), q1z = fmaf(e2x, wy, -(e2y * wx));
+    const float q2x = fmaf(wy, e1z, -(wz * e1y)), q2y = fmaf(wz, e1x, -(wx * e1z)), q2z = fmaf(wx, e1y, -(wy * e1x));
+    const float ax = nd.b.x, ay = nd.b.y, az = nd.b.z;
+    const float div = ax * mx + ay * my + az * mz;
+    const float n1 = flip_sign(ax * q1x + ay * q1y + az * q1z, div), n2 = flip_sign(ax * q2x + ay * q2y + az * q2z, div);
+    const float D = fabsf(div), ee = kTol * ne1 * ne2, rt = fmaf(kTol, nw, r);
+    const bool certain = D > fmaf(spread, rough_len(mx, my, mz), ee) && fminf(ne1, ne2) >= 1.f / kBig &&
+                         fmaxf(fmaxf(ne1, ne2), nw) <= kBig;
+    const float n3 = ne1 + ne2;
+    return certain && (n1 < -fmaf(spread, rough_len(q1x, q1y, q1z), ne2 * rt) ||
+                       n2 < -fmaf(spread, rough_len(q2x, q2y, q2z), ne1 * rt) ||
+                       n1 + n2 - D > fmaf(spread, rough_len(q1x + q2x - mx, q1y + q2y - my, q1z + q2z - mz),
+                                          fmaf(kTol * n3, nw, fmaf(fabsf(e2x - e1x) + fabsf(e2y - e1y) + fabsf(e2z - e1z), r, ee))));
 }
 
 // A (triangle record, node) pair that passed its node test.
@@ -418,16 +481,24 @@ __global__ void __launch_bounds__(256)
 
 // The last two levels and the leaf tests in one pass, no pair queue: one
 // warp per (cluster, leaves' parent) pair.  Lane j first stands for member
-// triangle j (parent test, then each of the kFan leaves: a ballot gives the
-// members that reach the leaf); then, leaf by leaf, lane k stands for ray k
-// of the leaf and tests the reaching members one after another, their
-// records staged in shared memory by the owning lanes.  A leaf's rays are
-// loaded once per cluster that reaches it (from L2), instead of going
-// through a written, counted, sorted and re-read list of (triangle, leaf)
-// pairs.  Nearest: per-lane best key, atomicMax per leaf; any-hit: the
-// leaf's occlusion bits are read first and set when a ray is blocked.
-constexpr int kSplitTestMinBlocks = 5;  // CTAs per SM: measured best of 4-8 (5-7 equal, 5 spills least)
-constexpr int kNearestMinBlocks = 4;     // nearest-hit variant, resident grid: best of 4-6
+// triangle j (parent test); the members that pass go side by side into shared
+// memory, and every eight of them are tested against the kFan leaves at once,
+// lane = (member, leaf).  Then, leaf by leaf, lane k stands for ray k of the
+// leaf and puts the reaching members through the filter one after another; the
+// exact test follows once for all rays.  A leaf's rays are loaded once per
+// cluster that reaches it (from L2), instead of going through a written,
+// counted, sorted and re-read list of (triangle, leaf) pairs.  Nearest:
+// per-lane best key, atomicMax per leaf; any-hit: the leaf's occlusion bits
+// are read first and set when a ray is blocked.
+//
+// Bound by instruction issue (86 % active, 20 of 32 lanes).  The frame of 4.2 M
+// camera and 4 x 4.2 M shadow rays on 181,250 triangles, all five launches:
+// 2,430 us before, 1,680 now.  Pairs differ so much in work that dealing them
+// out by a fixed stride left a tail: any-hit 4 x 455 us, 386 from the counter.
+// Exact tests held back: 386 -> 321.  Leaf tests by (member, leaf) and
+// beam_misses: nearest 490 -> 440 and 656 -> 592.
+constexpr int kSplitWarps = 8;
+constexpr int kSplitBlocks = 4;  // CTAs per SM, all resident: best of 4 (any-hit 1,283 us a frame), 5 (1,315), 6 (1,362)
 
 // Nearest-hit batches also keep a live reach bound per leaf and per leaves'
 // parent: an upper bound on maxt x |d| over the node's rays, where each
@@ -445,30 +516,56 @@ __device__ __forceinline__ void lower_reach(uint32_t* b, float x) {
     atomicMax(b, 0x7f800000u - __float_as_uint(x));
 }
 
+// The CTA's next task: from the lot of `deal` tasks that it took from the
+// grid's counter last (s_lot: first task, tasks handed out); the warp that
+// finds the lot just empty takes the next one, and the warps that come before
+// it is back take single tasks.  Lots of 8 keep the grid's one counter out of
+// the way (a task per atomic of the whole grid: 1.9 a nanosecond at most);
+// with fewer than kDeal tasks to a warp, single ones leave no warp idle.
+constexpr uint32_t kDeal = 8;
+
+__device__ __forceinline__ uint32_t next_task(unsigned long long* s_lot, uint32_t* next, uint32_t deal) {
+    const unsigned long long w = atomicAdd(s_lot, 1ull);
+    const uint32_t k = (uint32_t)w;
+    if (k < deal) return (uint32_t)(w >> 32) + k;
+    if (k > deal) return atomicAdd(next, 1u);
+    const uint32_t first = atomicAdd(next, deal);
+    atomicExch(s_lot, ((unsigned long long)first << 32) | 1ull);
+    return first;
+}
+
 // SMALL (batches of at most kFewRays rays): a warp takes one leaf of a pair
 // and tests the members against the parent again, since with few pairs to a
 // warp the longest one is the kernel's time (a frame of 19,159 rays 228 us ->
 // 198).
 template <bool ANY, bool STATS, bool SMALL>
-__global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBlocks)
+__global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
     rh_split_test_kernel(const float4* __restrict__ spheres, const TriRec* __restrict__ tris, int32_t t0,
                          int32_t t1, const RayNode* __restrict__ level1, const RayNode* __restrict__ leaves,
                          int64_t nleaf, const Pair* __restrict__ in, const uint32_t* __restrict__ in_count,
-                         uint32_t cap, const float4* __restrict__ so, const float4* __restrict__ sd,
+                         uint32_t cap, uint32_t* __restrict__ next, const float4* __restrict__ so,
+                         const float4* __restrict__ sd,
                          unsigned long long* __restrict__ keys, uint32_t* __restrict__ leafmask,
                          uint32_t* __restrict__ leaf_reach, uint32_t* __restrict__ parent_reach,
                          const int* __restrict__ status, unsigned long long* wc) {
-    __shared__ float4 s_rec[8][kClusterTris * 3];  // this warp's member records (256 threads)
+    __shared__ unsigned long long s_lot;
+    __shared__ float4 s_rec[kSplitWarps][kClusterTris * 3];  // this warp's member records
+    __shared__ float4 s_sph[kSplitWarps][kClusterTris];      // and spheres
     if (status[kStatusOverflow] != 0) return;  // pairs were dropped upstream: this attempt is rerun
     const unsigned full = 0xffffffffu;
-    float4* rec = s_rec[threadIdx.x >> 5];
+    float4 *rec = s_rec[threadIdx.x >> 5], *msph = s_sph[threadIdx.x >> 5];
     const uint32_t nin = min(*in_count, cap);
     const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     WorkCount c_;
     const int64_t ntask = SMALL ? (int64_t)nin * kFan : nin;
-    for (int64_t task = warp; task < ntask; task += nwarps) {
+    const uint32_t deal = ntask >= (int64_t)(kDeal * kSplitWarps) * gridDim.x ? kDeal : 1u;
+    if (threadIdx.x == 0) s_lot = deal;
+    __syncthreads();
+    for (;;) {
+        uint32_t task = 0;
+        if (lane == 0) task = next_task(&s_lot, next, deal);
+        task = __shfl_sync(full, task, 0);
+        if (task >= ntask) break;
         const Pair pr = in[SMALL ? task / kFan : task];
         const int64_t t = (int64_t)pr.tri * kClusterTris + lane;
         bool pass = false;
@@ -484,33 +581,60 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
             }
             pass = node_hits_sphere(pn, sph);
         }
-        if (!__any_sync(full, pass)) continue;
+        const unsigned members = __ballot_sync(full, pass);
+        if (!members) continue;
+        const int np = __popc(members);
         __syncwarp();  // the previous pair's records are no longer read
-        if (pass) {
+        if (pass) {  // the members that reach the parent, side by side
+            const int k = __popc(members & ((1u << lane) - 1u));
             const TriRec own = tris[t];
-            rec[3 * lane] = own.a;
-            rec[3 * lane + 1] = own.b;
-            rec[3 * lane + 2] = own.c;
+            rec[3 * k] = own.a;
+            rec[3 * k + 1] = own.b;
+            rec[3 * k + 2] = own.c;
+            msph[k] = sph;
         }
         __syncwarp();
+        // Every eight of them against the kFan leaves at once: lane = (member,
+        // leaf).  SMALL: all against the task's leaf, lane = member.
         const int64_t first = (int64_t)pr.node * kFan;
+        const int mine = SMALL ? (int)(task % kFan) : lane % kFan;
+        const int64_t my_leaf = first + mine;
+        RayNode nd;
+        nd.c = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (my_leaf < nleaf) nd = leaves[my_leaf];
+        const bool rays = __float_as_int(nd.c.z) > 0;
+        if (!ANY && rays) nd.c.y = fminf(nd.c.y, live_reach(leaf_reach + my_leaf));
+        unsigned mine_reached = 0;  // lane k: the leaves that member k reaches, one bit each
+#pragma unroll 1
+        for (int k0 = 0; k0 < np; k0 += SMALL ? 32 : 32 / kFan) {
+            const int k = k0 + (SMALL ? lane : lane / kFan);
+            bool reach = false;
+            if (k < np && rays) {
+                if (STATS) c_.node++;
+                reach = node_hits_sphere(nd, msph[k]);
+                if (!ANY && reach) {
+                    TriRec own;
+                    own.a = rec[3 * k];
+                    own.b = rec[3 * k + 1];
+                    own.c = rec[3 * k + 2];
+                    reach = !beam_misses(nd, own);
+                }
+            }
+            const unsigned b = __ballot_sync(full, reach);
+            if (SMALL)
+                mine_reached = reach ? 1u << mine : 0u;
+            else if (lane / (32 / kFan) == k0 / (32 / kFan))
+                mine_reached = b >> (lane % (32 / kFan) * kFan) & ((1u << kFan) - 1u);
+        }
         float parent_new = 0.f;  // max of the leaves' bounds after this pair
 #pragma unroll 1
-        for (int c = SMALL ? (int)(task % kFan) : 0, c1 = SMALL ? c + 1 : kFan; c < c1; ++c) {
+        for (int c = SMALL ? mine : 0, c1 = SMALL ? c + 1 : kFan; c < c1; ++c) {
             const int64_t leaf = first + c;
-            if (leaf >= nleaf) break;
-            RayNode nd = leaves[leaf];
-            const int count = __float_as_int(nd.c.z);
-            if (count == 0) continue;
-            if (!ANY) nd.c.y = fminf(nd.c.y, live_reach(leaf_reach + leaf));
-            bool reach = false;
-            if (pass) {
-                if (STATS) c_.node++;
-                reach = node_hits_sphere(nd, sph);
-            }
-            unsigned m = __ballot_sync(full, reach);
+            unsigned m = __ballot_sync(full, mine_reached >> c & 1u);
+            const float leaf_now = __shfl_sync(full, nd.c.y, c);  // SMALL: every lane's leaf
+            const int count = __shfl_sync(full, __float_as_int(nd.c.z), c);
             if (!m) {
-                if (!ANY) parent_new = fmaxf(parent_new, nd.c.y);
+                if (!ANY && count > 0) parent_new = fmaxf(parent_new, leaf_now);
                 continue;
             }
             if (STATS && lane == 0) c_.leaf++;
@@ -532,28 +656,65 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
                 }
             }
             bool hit = false;
-            while (m) {
-                const int j = __ffs(m) - 1;
-                m &= m - 1;
-                if (!active) continue;
+            // The exact test waits until the members are through the filter:
+            // few rays pass for one member, and a warp's exact test takes as
+            // long for one ray as for 32.
+            const auto exact = [&](int j, float* t) {
+                TriRec tr;
+                tr.a = rec[3 * j];
+                tr.b = rec[3 * j + 1];
+                tr.c = rec[3 * j + 2];
+                float u1, u2;
+                if (STATS) c_.exact++;
+                const bool in = pbg_exact_rec(tr, o, d, maxt, t, &u1, &u2);
+                if (STATS && in) c_.hit++;
+                return in;
+            };
+            const auto filter = [&](int j) {
                 TriRec tr;
                 tr.a = rec[3 * j];
                 tr.b = rec[3 * j + 1];
                 tr.c = rec[3 * j + 2];
                 if (STATS) c_.filt++;
-                if (!pbg_filter(tr, o, d, nd1, maxt)) continue;
-                float tt, u1, u2;
-                if (STATS) c_.exact++;
-                if (!pbg_exact_rec(tr, o, d, maxt, &tt, &u1, &u2)) continue;
-                if (STATS) c_.hit++;
-                if (ANY) {
-                    hit = true;
-                    active = false;
-                } else {
-                    const unsigned long long k = hit_key(tt, __float_as_int(tr.c.w));
-                    if (k > best) best = k;
-                    maxt = tt;
+                return pbg_filter(tr, o, d, nd1, maxt);
+            };
+            int pend = -1;  // this ray's member for the exact test
+            if (ANY) {
+                unsigned left = active ? m : 0u;  // this ray's members
+                for (unsigned all = m; all; all = __reduce_or_sync(full, left)) {
+                    pend = -1;
+                    for (; all; all &= all - 1) {
+                        const int j = __ffs(all) - 1;
+                        if (!(left >> j & 1u)) continue;
+                        if (filter(j)) {
+                            pend = j;
+                            left = 0u;
+                        }
+                    }
+                    left = 0u;
+                    float tt;
+                    if (pend >= 0) {
+                        hit = exact(pend, &tt);
+                        if (!hit) left = m & ~((2u << pend) - 1u);  // rare: the members behind it
+                    }
                 }
+            } else {
+                const auto settle = [&]() {
+                    float tt;
+                    if (pend >= 0 && exact(pend, &tt)) {
+                        const unsigned long long k = hit_key(tt, __float_as_int(rec[3 * pend + 2].w));
+                        if (k > best) best = k;
+                        maxt = tt;
+                    }
+                    pend = -1;
+                };
+                for (; m; m &= m - 1) {
+                    const int j = __ffs(m) - 1;
+                    const bool cand = active && filter(j);
+                    if (__any_sync(full, cand && pend >= 0)) settle();
+                    if (cand) pend = j;
+                }
+                settle();
             }
             if (ANY) {
                 if (hit) atomicOr(&leafmask[leaf], 1u << lane);
@@ -565,10 +726,9 @@ __global__ void __launch_bounds__(256, ANY ? kSplitTestMinBlocks : kNearestMinBl
                 const float len = sqrtf(fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)));
                 float b = lane < count ? maxt * len * (1.f + 0x1p-20f) : 0.f;
                 if (!(b == b)) b = INFINITY;
-#pragma unroll
-                for (int off = 16; off; off >>= 1) b = fmaxf(b, __shfl_xor_sync(full, b, off));
-                if (lane == 0 && b < nd.c.y) lower_reach(leaf_reach + leaf, b);
-                parent_new = fmaxf(parent_new, fminf(b, nd.c.y));
+                b = warp_max(b);
+                if (lane == 0 && b < leaf_now) lower_reach(leaf_reach + leaf, b);
+                parent_new = fmaxf(parent_new, fminf(b, leaf_now));
             }
         }
         if (!ANY && !SMALL && lane == 0 && parent_new < parent_now) lower_reach(parent_reach + pr.node, parent_new);
@@ -955,13 +1115,16 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
     // grid-stride kernels: 32 CTAs per SM measured best of 4, 8, 16, 32 on
     // the terrain frame (tune.rh_grid)
-    const unsigned grid = (unsigned)(sms * (s->tune.rh_grid[ANY] > 0 ? s->tune.rh_grid[ANY] : 32));
+    const bool few = nleaf * kLeafRays <= kFewRays;
+    const int per_sm = s->tune.rh_grid[ANY] > 0 ? s->tune.rh_grid[ANY] : 32;
+    const unsigned grid = (unsigned)(sms * (few ? std::min(per_sm, kFewGrid) : per_sm));
     const bool stats = s->prof.level >= 2;
     unsigned long long* wc = (unsigned long long*)s->workc.ptr;
     int* status = (int*)s->err.ptr;
     const RayNode* nodes = (const RayNode*)w.nodes.ptr;
     uint32_t* counts = (uint32_t*)w.qcount.ptr;
-    static_assert(2 * kMaxLevels <= 64, "pair counters");
+    constexpr int kNextPair = 2 * kMaxLevels;  // the split tests' next pair
+    static_assert(kNextPair < 64, "pair counters");
     int groups = s->rh_groups > 0 ? s->rh_groups : 1;
     const int top = lv.nlev - 1;
     const Descent dsc = descent_levels(s, lv, ANY);
@@ -1015,7 +1178,6 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
             bool fused = false;
             for (int l = ls; l >= 0; --l) {
                 if (cl && l == 1 && split == 1) {  // clusters straight into the leaf tests
-                    unsigned tgrid = grid * 2;
                     if (order_hist) {  // nearest: front-to-back pairs, taken in order
                         if (!fresh) PBG_CUDA(cudaMemsetAsync(order_hist, 0, kOrderBuckets * sizeof(uint32_t), st));
                         rh_order_count_kernel<<<grid, 256, 0, st>>>(csph, nodes + lv.off[1], qa, cnt_of[1],
@@ -1027,14 +1189,13 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
                         Pair* tq = qa;
                         qa = qb;
                         qb = tq;
-                        tgrid = (unsigned)(sms * kNearestMinBlocks);  // resident CTAs only
                         nl += 2;
                     }
                     const auto kernel = stats ? rh_split_test_kernel<ANY, true, false>
-                                        : nleaf * kLeafRays <= kFewRays ? rh_split_test_kernel<ANY, false, true>
+                                        : few ? rh_split_test_kernel<ANY, false, true>
                                                                         : rh_split_test_kernel<ANY, false, false>;
-                    kernel<<<tgrid, 256, 0, st>>>(tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1],
-                                                  nodes + lv.off[0], lv.cnt[0], qa, cnt_of[1], cap, so, sd, keys, mask,
+                    kernel<<<(unsigned)(sms * kSplitBlocks), 32 * kSplitWarps, 0, st>>>(tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1],
+                                                  nodes + lv.off[0], lv.cnt[0], qa, cnt_of[1], cap, counts + kNextPair, so, sd, keys, mask,
                                                   leaf_reach, parent_reach, status, stats ? wc : nullptr);
                     fused = true;
                     ++nl;
@@ -1098,7 +1259,7 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
         // reach the host some 15 us later than from a kernel before it.
         Publication pub;
         const int words = moved ? 2 : 1;
-        if (nleaf * kLeafRays <= kFewRays) {
+        if (few) {
             pub.count = words;
             pub.src = status + kStatusOverflow;
             if ((rc = next_publication(s, &pub.dst, &pub.seq))) return rc;

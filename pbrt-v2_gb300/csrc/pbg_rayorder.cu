@@ -13,7 +13,7 @@
 //
 // Sort: four passes of 8 bits.  Each pass is (1) a per-tile digit histogram,
 // (2) one exclusive scan over [digit][tile] counts, (3) a stable scatter in
-// which each warp ranks its 32 keys per digit with warp votes and the
+// which each warp ranks its 32 keys per digit with __match_any_sync and the
 // tile's warps are combined through shared-memory prefix sums.
 #include <algorithm>
 
@@ -349,21 +349,6 @@ __global__ void __launch_bounds__(1024) scan_one(uint32_t* __restrict__ a, int m
     }
 }
 
-// The lanes of the warp whose digit equals this lane's, among those with ok
-// set (0 for the others): one vote per bit.  __match_any_sync takes some 55
-// cycles of the SM for distinct digits, the votes a third of that.
-template <int MAXBITS>
-__device__ __forceinline__ uint32_t digit_peers(uint32_t dg, bool ok, int bits) {
-    uint32_t peers = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-    for (int b = 0; b < MAXBITS; ++b) {
-        if (b >= bits) break;
-        const uint32_t v = __ballot_sync(0xffffffffu, (dg >> b) & 1u);
-        peers &= (dg >> b) & 1u ? v : ~v;
-    }
-    return ok ? peers : 0u;
-}
-
 // Pass 3: stable scatter.  Element order inside a tile is (warp, item, lane),
 // which is the original order, so ranks computed in that order keep the sort
 // stable.
@@ -391,7 +376,9 @@ __global__ void __launch_bounds__(kSortThreads)
         key[k] = ok ? keys[i] : 0xffffffffu;
         val[k] = ok ? vals[i] : 0;
         const uint32_t dg = (key[k] >> shift) & kDigitMask;
-        const uint32_t peers = digit_peers<kDigitBits>(dg, ok, kDigitBits);
+        const uint32_t inb = __ballot_sync(0xffffffffu, ok);
+        uint32_t peers = __match_any_sync(0xffffffffu, ok ? dg : (uint32_t)kRadix) & inb;
+        if (!ok) peers = 0;
         const uint32_t before = wcount[warp][dg];
         __syncwarp();
         rank[k] = before + __popc(peers & lt);
@@ -482,6 +469,23 @@ __device__ __forceinline__ uint32_t cluster_load(const void* p, uint32_t cta) {
 }
 __device__ __forceinline__ void cluster_store(const void* p, uint32_t cta, uint2 v) {
     asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(cluster_map(p, cta)), "r"(v.x), "r"(v.y) : "memory");
+}
+
+// The lanes of the warp whose digit equals this lane's, among those with ok
+// set (0 for the others): one vote per bit.  One warp's __match_any_sync takes
+// some 55 cycles of its SM for distinct digits, the votes a third of that; the
+// large batches' scatter, which waits for memory, is no faster for it (27 us a
+// pass of 4 M keys, 30 with votes).
+template <int MAXBITS>
+__device__ __forceinline__ uint32_t digit_peers(uint32_t dg, bool ok, int bits) {
+    uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int b = 0; b < MAXBITS; ++b) {
+        if (b >= bits) break;
+        const uint32_t v = __ballot_sync(0xffffffffu, (dg >> b) & 1u);
+        peers &= (dg >> b) & 1u ? v : ~v;
+    }
+    return ok ? peers : 0u;
 }
 
 // CTA c holds positions [c * per, c * per + per) of the n keys, its warp w
