@@ -142,31 +142,46 @@ struct WalkHit {
     int32_t prim;
 };
 
-// Tests records [start, start + cnt); returns true when an any-hit query is done.
+// The exact test of record `rec` and its effect on the hit; returns true when
+// an any-hit query is done.
+template <bool ANY, bool STATS>
+__device__ __forceinline__ bool test_exact(const TriRec* __restrict__ tris, int32_t rec, float4 o, float4 d,
+                                           WalkHit& h, WorkCount& wc) {
+    const TriRec tr = tris[rec];
+    float tt, u1, u2;
+    if (STATS) wc.exact++;
+    if (!pbg_exact_rec(tr, o, d, h.t, &tt, &u1, &u2)) return false;
+    if (STATS) wc.hit++;
+    const int32_t id = __float_as_int(tr.c.w);
+    if (ANY) {
+        h.prim = id;
+        return true;
+    }
+    if (tt < h.t || id > h.prim) {
+        h.t = tt;
+        h.prim = id;
+        h.b1 = u1;
+        h.b2 = u2;
+    }
+    return false;
+}
+
+// Tests records [start, start + cnt); returns true when an any-hit query is
+// done.  A record that passes the filter waits for the next that does, or for
+// the last record: few of the warp's rays pass at one record, and its exact
+// test takes as long for one ray as for 32 (ordered walk 666 -> 642 us, 500
+// picking rays 19.2 -> 18.4).
 template <bool ANY, bool STATS>
 __device__ __forceinline__ bool test_run(const TriRec* __restrict__ tris, int32_t start, int32_t cnt,
                                          float4 o, float4 d, float nd, WalkHit& h, WorkCount& wc) {
+    int32_t pend = -1;
     for (int32_t k = 0; k < cnt; ++k) {
-        const TriRec tr = tris[start + k];
         if (STATS) wc.filt++;
-        if (!pbg_filter(tr, o, d, nd, h.t, STATS ? &wc.filt2 : nullptr)) continue;
-        float tt, u1, u2;
-        if (STATS) wc.exact++;
-        if (!pbg_exact_rec(tr, o, d, h.t, &tt, &u1, &u2)) continue;
-        if (STATS) wc.hit++;
-        const int32_t id = __float_as_int(tr.c.w);
-        if (ANY) {
-            h.prim = id;
-            return true;
-        }
-        if (tt < h.t || id > h.prim) {
-            h.t = tt;
-            h.prim = id;
-            h.b1 = u1;
-            h.b2 = u2;
-        }
+        if (!pbg_filter(tris[start + k], o, d, nd, h.t, STATS ? &wc.filt2 : nullptr)) continue;
+        if (pend >= 0 && test_exact<ANY, STATS>(tris, pend, o, d, h, wc)) return true;
+        pend = start + k;
     }
-    return false;
+    return pend >= 0 && test_exact<ANY, STATS>(tris, pend, o, d, h, wc);
 }
 
 // The walk.  h.t starts at the ray's maxt and h.prim at -1.  ORDERED: the

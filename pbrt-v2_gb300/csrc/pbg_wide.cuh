@@ -65,6 +65,7 @@ struct CoopWarp {
     float ht[32], nd[32], t[32], b1[32], b2[32];
     uint32_t m1[32], m2[32], m3[32];
     int32_t base1[32], base2[32], base3[32], off[32], occluder[32];
+    int2 queue[64];              // (owner, record) for the exact test
 };
 
 // Children in visiting order: slot ^ visit_order(octant).  Nearest hits go
@@ -171,11 +172,11 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
             const bool searching = has && tmask == 0 && rcnt == 0;
             if (!__any_sync(full, searching)) break;
             // walk 6: the tests are dealt over the warp, so they need not
-            // wait for the last searching lane: once four lanes hold two
-            // nodes' triangles the warp tests (64 scenes 5.95 / 5.95 / 5.98 /
-            // 6.03 ms and path frame 18.9 / 18.9 / 19.0 / 19.2 ms for 3, 4, 6
-            // and 8 such lanes)
-            if (COOP && __popc(__ballot_sync(full, has && tmask2 != 0)) >= 4) break;
+            // wait for the last searching lane: once six lanes hold two
+            // nodes' triangles the warp tests (64 scenes 5.28 / 5.21 / 5.16 /
+            // 5.15 / 5.16 ms and path frame 17.6 / 17.5 / 17.4 / 17.5 / 17.7 ms
+            // for 3, 4, 6, 8 and 12 such lanes)
+            if (COOP && __popc(__ballot_sync(full, has && tmask2 != 0)) >= 6) break;
             // any-hit rays end at very different times: with 16 lanes idle
             // the warp takes new rays (direct lighting 966 -> 933 us; for
             // nearest hits 18.87 -> 19.12 ms, so not there)
@@ -328,13 +329,18 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                     cw.key[lane] = own;
                 }
                 __syncwarp();
-                for (int g0 = 0; g0 < total; g0 += 32) {
+                // Pairs that pass the filter queue for the exact test, which
+                // runs for 32 of them or after the last round: some four of a
+                // round's 32 pass, and it takes as long for one as for 32
+                // (path bounces 938 -> 788 us, path frame 18.9 -> 17.5 ms, 64
+                // scenes 5.93 -> 5.19 ms).
+                int queued = 0;
+                for (int g0 = 0; g0 < total || queued > 0; g0 += 32) {
                     const int g = g0 + lane;
-                    int ci = -1;
-                    unsigned long long ck = 0ull;
-                    float ct = 0.f, cu1 = 0.f, cu2 = 0.f;
+                    bool cand = false;
+                    int i = 0;  // the owner: the last lane whose first pair is <= g
+                    int32_t rec = 0;
                     if (g < total) {
-                        int i = 0;  // the owner: the last lane whose first pair is <= g
 #pragma unroll
                         for (int step = 16; step; step >>= 1)
                             if (cw.off[i + step] <= g) i += step;
@@ -343,31 +349,39 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                         const int n1 = __popc(m1);
                         const uint32_t m2v = cw.m2[i];
                         const int n2 = __popc(m2v);
-                        const int32_t rec = k < n1        ? cw.base1[i] + (int)__fns(m1, 0, k + 1)
-                                            : k < n1 + n2 ? cw.base2[i] + (int)__fns(m2v, 0, k - n1 + 1)
-                                                          : cw.base3[i] + (int)__fns(cw.m3[i], 0, k - n1 - n2 + 1);
+                        rec = k < n1        ? cw.base1[i] + (int)__fns(m1, 0, k + 1)
+                              : k < n1 + n2 ? cw.base2[i] + (int)__fns(m2v, 0, k - n1 + 1)
+                                            : cw.base3[i] + (int)__fns(cw.m3[i], 0, k - n1 - n2 + 1);
                         if (!ANY || cw.key[i] == 0ull) {
-                            const float4 oo = cw.o[i], dd = cw.d[i];
-                            const float bound = cw.ht[i];
-                            const TriRec tr = (Src::kSet ? cw.tris[i] : src.tris(L))[rec];
                             if (STATS) wc.filt++;
-                            if (pbg_filter(tr, oo, dd, cw.nd[i], bound, STATS ? &wc.filt2 : nullptr)) {
-                                float tt, u1, u2;
-                                if (STATS) wc.exact++;
-                                if (pbg_exact_rec(tr, oo, dd, bound, &tt, &u1, &u2)) {
-                                    if (STATS) wc.hit++;
-                                    const int32_t id = __float_as_int(tr.c.w);
-                                    if (ANY) {
-                                        cw.key[i] = 1ull;
-                                        cw.occluder[i] = id;
-                                    } else {
-                                        ci = i;
-                                        ck = hit_key(tt, id);
-                                        ct = tt;
-                                        cu1 = u1;
-                                        cu2 = u2;
-                                        atomicMax(&cw.key[i], ck);
-                                    }
+                            cand = pbg_filter((Src::kSet ? cw.tris[i] : src.tris(L))[rec], cw.o[i], cw.d[i], cw.nd[i],
+                                              cw.ht[i], STATS ? &wc.filt2 : nullptr);
+                        }
+                    }
+                    const unsigned cm = __ballot_sync(full, cand);
+                    if (cand) cw.queue[queued + __popc(cm & lt)] = make_int2(i, rec);
+                    queued += __popc(cm);
+                    if (queued == 0 || (queued < 32 && g0 + 32 < total)) continue;
+                    __syncwarp();
+                    const int take = min(queued, 32);
+                    unsigned long long ck = 0ull;
+                    float ct = 0.f, cu1 = 0.f, cu2 = 0.f;
+                    int ci = -1;
+                    if (lane < take) {
+                        const int2 e = cw.queue[lane];
+                        if (!ANY || cw.key[e.x] == 0ull) {
+                            const TriRec tr = (Src::kSet ? cw.tris[e.x] : src.tris(L))[e.y];
+                            if (STATS) wc.exact++;
+                            if (pbg_exact_rec(tr, cw.o[e.x], cw.d[e.x], cw.ht[e.x], &ct, &cu1, &cu2)) {
+                                if (STATS) wc.hit++;
+                                const int32_t id = __float_as_int(tr.c.w);
+                                if (ANY) {
+                                    cw.key[e.x] = 1ull;
+                                    cw.occluder[e.x] = id;
+                                } else {
+                                    ci = e.x;
+                                    ck = hit_key(ct, id);
+                                    atomicMax(&cw.key[ci], ck);
                                 }
                             }
                         }
@@ -378,6 +392,11 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                         cw.b1[ci] = cu1;
                         cw.b2[ci] = cu2;
                     }
+                    int2 behind = make_int2(0, 0);
+                    queued -= take;
+                    if (lane < queued) behind = cw.queue[32 + lane];
+                    __syncwarp();
+                    if (lane < queued) cw.queue[lane] = behind;
                     __syncwarp();
                 }
                 if (mine) {
@@ -399,22 +418,33 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
             tmask = 0;
             tmask2 = 0;
             tmask3 = 0;
-        } else if (has && (tmask != 0 || tmask2 != 0 || rcnt != 0)) {
-            if (STATS) wc.leaf++;
+        } else {
+            const bool mine = has && (tmask != 0 || tmask2 != 0 || rcnt != 0);
+            if (STATS && mine) wc.leaf++;
             bool done = false;
-            if (rcnt) {
+            if (mine && rcnt) {
                 done = test_run<ANY, STATS>(src.tris(L), 0, rcnt, o, d, nd, h, wc);
                 rcnt = 0;
             }
-            while (!done && tmask) {
-                const int b = __ffs(tmask) - 1;
-                tmask &= tmask - 1u;
-                done = test_run<ANY, STATS>(src.tris(L), tbase + b, 1, o, d, nd, h, wc);
-            }
-            while (!done && tmask2) {
-                const int b = __ffs(tmask2) - 1;
-                tmask2 &= tmask2 - 1u;
-                done = test_run<ANY, STATS>(src.tris(L), tbase2 + b, 1, o, d, nd, h, wc);
+            // every lane on to its next record that passes the filter, then
+            // the exact test for all of them together
+            for (;;) {
+                int32_t cand = -1;
+                if (mine && !done) {
+                    while (cand < 0 && (tmask | tmask2) != 0) {
+                        const bool one = tmask != 0;
+                        const uint32_t m = one ? tmask : tmask2;
+                        const int32_t rec = (one ? tbase : tbase2) + __ffs(m) - 1;
+                        if (one)
+                            tmask = m & (m - 1u);
+                        else
+                            tmask2 = m & (m - 1u);
+                        if (STATS) wc.filt++;
+                        if (pbg_filter(src.tris(L)[rec], o, d, nd, h.t, STATS ? &wc.filt2 : nullptr)) cand = rec;
+                    }
+                }
+                if (!__any_sync(full, cand >= 0)) break;
+                if (cand >= 0) done = test_exact<ANY, STATS>(src.tris(L), cand, o, d, h, wc);
             }
             tmask = 0;
             tmask2 = 0;
