@@ -1393,13 +1393,24 @@ int pbg_hit_geometry(pbg_scene* s, const pbg_rays* r, const pbg_hits* h, int64_t
         (rc = ensure(w.b1, (size_t)n * 4)) || (rc = ensure(w.b2, (size_t)n * 4)) ||
         (rc = ensure(w.geo, (size_t)n * 14 * 4)))
         return rc;
-    PBG_CUDA(cudaMemcpyAsync(w.prim.ptr, h->prim, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
-    PBG_CUDA(cudaMemcpyAsync(w.t.ptr, h->t, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
-    PBG_CUDA(cudaMemcpyAsync(w.b1.ptr, h->b1, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
-    PBG_CUDA(cudaMemcpyAsync(w.b2.ptr, h->b2, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
-    rc = hit_geometry(s, o, d, (const int32_t*)w.prim.ptr, (const float*)w.t.ptr,
-                      (const float*)w.b1.ptr, (const float*)w.b2.ptr, n, (float*)w.geo.ptr,
-                      s->stream);
+    // The hits are read in place where the GPU can address them (640 x 640
+    // hits: 390 us by copies, 332 so); the results, in pages that are often
+    // new, go back by the copy engine (a kernel's stores: 494 us).
+    const int32_t* prim = (const int32_t*)device_view(s->device, h->prim);
+    const float* t = (const float*)device_view(s->device, h->t);
+    const float* b1 = (const float*)device_view(s->device, h->b1);
+    const float* b2 = (const float*)device_view(s->device, h->b2);
+    if (!prim || !t || !b1 || !b2) {
+        PBG_CUDA(cudaMemcpyAsync(w.prim.ptr, h->prim, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
+        PBG_CUDA(cudaMemcpyAsync(w.t.ptr, h->t, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
+        PBG_CUDA(cudaMemcpyAsync(w.b1.ptr, h->b1, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
+        PBG_CUDA(cudaMemcpyAsync(w.b2.ptr, h->b2, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
+        prim = (const int32_t*)w.prim.ptr;
+        t = (const float*)w.t.ptr;
+        b1 = (const float*)w.b1.ptr;
+        b2 = (const float*)w.b2.ptr;
+    }
+    rc = hit_geometry(s, o, d, prim, t, b1, b2, n, (float*)w.geo.ptr, s->stream);
     if (rc) return rc;
     PBG_CUDA(cudaMemcpyAsync(out14, w.geo.ptr, (size_t)n * 14 * 4, cudaMemcpyDeviceToHost, s->stream));
     PBG_CUDA(cudaStreamSynchronize(s->stream));
