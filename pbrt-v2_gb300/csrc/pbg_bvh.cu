@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kPacketThreads)
             d = rd[ray];
         }
         const float ndd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
-        const RayInv ri{o.x, o.y, o.z, safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)};
+        const RayFma ri = ray_fma(o, d);  // direct lighting's camera rays 308 -> 301 us; the persistent walk is no faster for it
         WalkHit h{d.w, 0.f, 0.f, -1};
         bool done = !active;
         if (!done && unculled > 0) done = test_run<ANY, STATS>(tris, 0, unculled, o, d, ndd, h, wc);

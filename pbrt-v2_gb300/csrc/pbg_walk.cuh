@@ -92,6 +92,19 @@ __device__ __forceinline__ bool slab(const RayInv& r, float lx, float hx, float 
     return tn <= fmaf(fabsf(tf), kSlabWiden, tf);
 }
 
+// The same test with fused distances, a box's two planes of an axis in one
+// instruction.
+__device__ __forceinline__ bool slab(const RayFma& r, float lx, float hx, float ly, float hy,
+                                     float lz, float hz, float tmin, float tmax, float* tnear) {
+    const float2 tx = fma2(make_float2(lx, hx), make_float2(r.ix, r.ix), make_float2(r.cx, r.cx));
+    const float2 ty = fma2(make_float2(ly, hy), make_float2(r.iy, r.iy), make_float2(r.cy, r.cy));
+    const float2 tz = fma2(make_float2(lz, hz), make_float2(r.iz, r.iz), make_float2(r.cz, r.cz));
+    const float tn = fmax3(fminf(tx.x, tx.y), fminf(ty.x, ty.y), fmaxf(fminf(tz.x, tz.y), tmin));
+    const float tf = fmin3(fmaxf(tx.x, tx.y), fmaxf(ty.x, ty.y), fminf(fmaxf(tz.x, tz.y), tmax));
+    *tnear = tn;
+    return tn <= fmaf(fabsf(tf), kSlabWiden, tf);
+}
+
 // The walk's stack.  PACK: one 8-byte entry (one local load per pop) when
 // the scene allows it: a child reference, with a leaf's record start (below
 // 2^24) and triangle count (below 128) packed into one negative word, and
