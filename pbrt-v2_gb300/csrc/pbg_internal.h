@@ -79,7 +79,7 @@ struct Tunables {
     int naive_ctas = 16;     // naive: CTAs per SM the triangle splits aim for
     // rayhierarchy [any-hit]: nodes of the level the descent starts at (at
     // most), CTAs per SM of the grid-stride kernels
-    int rh_seed[2] = {256, 256};
+    int rh_seed[2] = {1024, 1024};
     int rh_grid[2] = {32, 32};
     int bvh_walk[2][2] = {{0, 0}, {0, 0}};  // ray-bvh [any-hit][incoherent]: 0 automatic, else pbg_params.walk's 1-6
 };

@@ -87,7 +87,7 @@ std::vector<Candidate> candidates(const pbg_scene* s) {
             for (int k : {4, 2, 8, 16}) out.push_back({{k, 0, 0}});
             break;
         case PBG_ACCEL_RAYHIERARCHY:
-            for (int seed : {256, 64, 1024})
+            for (int seed : {1024, 64, 256})
                 for (int grid : {32, 16}) out.push_back({{seed, grid, 0}});
             break;
         case PBG_ACCEL_RAYBVH:
