@@ -75,10 +75,10 @@ typedef struct pbg_params {
     int32_t walk;         /* ray-bvh traversal: 0 = automatic (what pbg_autotune
                            * chose for the batch class, else 6 for bounce
                            * batches -- nearest hit with a validity mask, and
-                           * the renderer's bounces >= 1 --; for the others of
-                           * 786,432 rays or more 4 nearest-hit, 5 any-hit, and
-                           * 6 below that, or 2 where the scene has no
-                           * eight-wide tree yet),
+                           * the renderer's bounces >= 1 --; for the others 4
+                           * nearest-hit from 786,432 rays, 5 any-hit from
+                           * 262,144, and 6 below that, or 2 where the scene
+                           * has no eight-wide tree yet),
                            * 1 = one thread per ray, 2 = persistent warps refilled
                            * from a ray counter, 3 = co-traversal of the ray
                            * hierarchy's 32-ray leaves with the BVH, one warp

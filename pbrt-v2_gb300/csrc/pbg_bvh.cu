@@ -422,7 +422,8 @@ static int walk_counter(pbg_scene* s, const QueueRef& q, unsigned long long** ne
 }
 
 // The walk of a batch class (hint 1: incoherent) of n rays.
-constexpr int64_t kPacketRays = 3 << 18;
+constexpr int64_t kPacketRays = 3 << 18;   // camera rays that pay for packets
+constexpr int64_t kOwnTestRays = 1 << 18;  // shadow rays that pay for walk 5
 static int choose_walk(const pbg_scene* s, bool any, int hint, int64_t n) {
     if (s->params.walk != 0) return s->params.walk;
     const int tuned = s->tune.bvh_walk[any ? 1 : 0][hint == 1 ? 1 : 0];
@@ -432,17 +433,21 @@ static int choose_walk(const pbg_scene* s, bool any, int hint, int64_t n) {
     // chip several times over; below that a packet's one dependent walk is the
     // whole time.  Measured on terrains of 20,000 and 181,250 triangles and
     // 1,024,000 triangles of spheres, us:
-    //   camera 500 rays      walk 4 217 / 288 / 370, 6  51 /  81 /  81, 2  60 / 90 / 90
-    //   camera 480,000       walk 4 154 / 274 / 425, 6 160 / 232 / 301
-    //   camera 1,048,576     walk 4 203 / 367 / 674, 6 271 / 439 / 672
-    //   shadow 500           walk 5  38 /  47 /  70, 6  33 /  41 /  65
-    //   shadow 480,000       walk 5  86 / 132 / 310, 6  90 / 130 / 268
-    //   shadow 1,048,576     walk 5 140 / 236 / 639, 6 150 / 242 / 550
-    //   shadow 4 to 8 M      walk 5 369 / 666 / 4337, 6 444 / 782 / 3868
-    // A scene that has traced only small camera batches has no eight-wide
-    // tree yet: walk 2 then, nearly as fast, instead of building one.
+    //   camera 500 rays      walk 4 224 / 300 / 386, 6  39 /  61 /  62, 2  52 / 81 / 80
+    //   camera 480,000       walk 4 145 / 249 / 419, 6 108 / 164 / 216, 2 132 / 218 / 297
+    //   camera 1,048,576     walk 4 188 / 351 / 670, 6 186 / 308 / 472, 2 226 / 363 / 631
+    //   camera 4,194,304     walk 4 431 / 702 / 1272, 6 589 / 979 / 1541
+    //   shadow 500           walk 5  34 /  35 /  59, 6  31 /  35 /  62
+    //   shadow 50,000        walk 5  45 /  53 /  99, 6  41 /  50 /  97
+    //   shadow 480,000       walk 5  65 /  96 / 227, 6  73 / 104 / 233
+    //   shadow 4,194,304     walk 5 271 / 474 / 1481, 6 354 / 597 / 1714
+    // The camera line is for several samples a pixel, whose packets are denser
+    // than the ones above: the 1,228,800 rays of a frame of 640 x 480 x 4 take
+    // packets in 876 us a frame, walk 6 in 897.  A scene that
+    // has traced only small camera batches has no eight-wide tree yet: walk 2
+    // then, instead of building one.
     if (hint == 1) return 6;
-    if (any) return n < kPacketRays ? 6 : 5;
+    if (any) return n < kOwnTestRays ? 6 : 5;
     return n >= kPacketRays ? 4 : s->wide_state > 0 ? 6 : 2;
 }
 

@@ -1,5 +1,5 @@
 """The walks that an untuned ray-bvh scene chooses by the batch's size: the
-same answers as one thread per ray on both sides of the line, before and after
+same answers as one thread per ray on both sides of the lines, before and after
 the scene has its eight-wide tree."""
 import numpy as np
 import pytest
@@ -11,10 +11,10 @@ from pbrt_gb300 import accel as A  # noqa: E402
 from pbrt_gb300 import scenes as S  # noqa: E402
 
 pytestmark = pytest.mark.gpu
-LINE = 3 << 18
+SHADOW, CAMERA = 1 << 18, 3 << 18  # the lines
 
 
-@pytest.mark.parametrize("n", [1, 33, LINE - 1, LINE])
+@pytest.mark.parametrize("n", [1, 33, SHADOW - 1, SHADOW, CAMERA - 1, CAMERA])
 def test_choice_by_size(gpu_lib, n):
     tris = S.terrain_icospheres(seed=2, grid=48, n_spheres=6)["tris"]
     side = int(np.ceil(np.sqrt(n)))
