@@ -11,11 +11,13 @@
 // direction whatever produced them.  Invalid rays get the key 0xffffffff and
 // sort to the end.
 //
-// Sort: four passes of 8 bits.  Each pass is (1) a per-tile digit histogram,
+// Sort (batches above 131,072 rays; smaller ones: sort_cluster_kernel, one
+// launch): four passes of 8 bits.  Each pass is (1) a per-tile digit histogram,
 // (2) one exclusive scan over [digit][tile] counts, (3) a stable scatter in
 // which each warp ranks its 32 keys per digit with __match_any_sync and the
 // tile's warps are combined through shared-memory prefix sums.
 #include <algorithm>
+#include <atomic>
 
 #include "pbg_curve.cuh"
 #include "pbg_internal.h"
@@ -642,19 +644,48 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     }
 }
 
-// One cluster sorts the n <= kClusterKeys keys of src into (keys_out, vals_out).
+// Per-device settings (cheap, idempotent): set on every call so that each
+// device the library launches on has them.
+static cudaError_t sort_cluster_attributes() {
+    const cudaError_t e = cudaFuncSetAttribute(sort_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(ClusterSmem));
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(sort_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+// Keys that one cluster of the device can sort: half where it has no room for
+// 16 CTAs (more than the portable size, so not promised).
+static int64_t cluster_keys(int device) {
+    static std::atomic<int> fits[64];  // 0 not asked yet, 1 no, 2 yes
+    if (device < 0 || device >= 64) return kClusterKeys / 2;
+    if (fits[device].load() == 0) {
+        cudaLaunchAttribute dims{};
+        dims.id = cudaLaunchAttributeClusterDimension;
+        dims.val.clusterDim.x = kClusterCtas;
+        dims.val.clusterDim.y = dims.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kClusterCtas);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.dynamicSmemBytes = sizeof(ClusterSmem);
+        cfg.attrs = &dims;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool ok = sort_cluster_attributes() == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, sort_cluster_kernel, &cfg) == cudaSuccess && clusters > 0;
+        if (!ok) cudaGetLastError();
+        fits[device].store(ok ? 2 : 1);
+    }
+    return fits[device].load() == 2 ? kClusterKeys : kClusterKeys / 2;
+}
+
+// One cluster sorts the n <= cluster_keys() keys of src into (keys_out, vals_out).
 static int sort_cluster(pbg_scene* s, const SortSource& src, int64_t n, int bits, uint32_t* keys_out, int32_t* vals_out,
                         cudaStream_t st) {
-    // a per-device setting (cheap, idempotent): set on every call so that each
-    // device the library launches on has it
-    PBG_CUDA(cudaFuncSetAttribute(sort_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(ClusterSmem)));
-    PBG_CUDA(cudaFuncSetAttribute(sort_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    PBG_CUDA(sort_cluster_attributes());
     // The most keys take the widest cluster; up to kClusterSmall, where an
     // 8-CTA cluster's barriers are the shorter part, half of it (frames of
     // 1,200 / 19,159 / 65,280 rays: 163 / 229 / 380 us with 8 CTAs, 172 / 228 /
     // 356 with 16).
-    const int ctas = n <= kClusterSmall ? kClusterCtas / 2 : kClusterCtas;
+    const int ctas = n <= kClusterSmall || cluster_keys(s->device) < kClusterKeys ? kClusterCtas / 2 : kClusterCtas;
     const int per = (int)(((n + ctas - 1) / ctas + 31) / 32 * 32);
     const int items = (per + kClusterThreads - 1) / kClusterThreads;
     if (src.mode == kKeysImage) {  // the keys' own bits, and one above them where invalid rays sort last
@@ -694,7 +725,7 @@ size_t radix_hist_words(int64_t n) {
 int radix_sort_pairs(pbg_scene* s, uint32_t* keys, int32_t* vals, uint32_t* keys_tmp, int32_t* vals_tmp,
                      uint32_t* hist, int64_t n, int bits, uint32_t** keys_out, int32_t** vals_out,
                      cudaStream_t st) {
-    if (n > 0 && n <= kClusterKeys) {
+    if (n > 0 && n <= cluster_keys(s->device)) {
         SortSource src;
         src.keys = keys;
         src.vals = vals;
@@ -795,7 +826,7 @@ int ray_sort(pbg_scene* s, const float4* o, const float4* d, const uint8_t* vali
         const bool comparable = was_cached && before[0] == w.origin_cache.ptr &&
                                 before[1] == w.osort_keys.ptr && before[2] == w.osort_perm.ptr &&
                                 before[3] == w.origin_valid.ptr;
-        if (!comparable && n <= kClusterKeys) {
+        if (!comparable && n <= cluster_keys(s->device)) {
             SortSource src;
             src.mode = kKeysOrigin;
             src.o = o;
@@ -848,7 +879,7 @@ int ray_sort(pbg_scene* s, const float4* o, const float4* d, const uint8_t* vali
         *perm = (const int32_t*)w.perm_tmp.ptr;
         if (sorted_keys) *sorted_keys = (const uint32_t*)w.mkeys_tmp.ptr;
         return PBG_OK;
-    } else if (n <= kClusterKeys) {
+    } else if (n <= cluster_keys(s->device)) {
         SortSource src;
         src.mode = s->image_w > 0 && n == s->image_w * s->image_h ? kKeysImage : kKeysMorton;
         src.o = o;
