@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kPacketThreads)
         int32_t node = 0;
         for (;;) {
             if (__all_sync(full, done)) break;
-            const BvhNode nd_ = nodes[node];
+            const BvhNode nd_ = load_node(nodes + node);
             float tn0 = 0.f, tn1 = 0.f;
             bool h0 = false, h1 = false;
             if (!done) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
                 if (!some && leaf_cnt == 0) finish();  // stack empty, nothing pending: done
                 continue;
             }
-            const BvhNode nn = nodes[node];
+            const BvhNode nn = load_node(nodes + node);
             if (STATS) wc.node += 2;
             float tn0, tn1;
             bool h0 = slab(ri, nn.n0.x, nn.n0.y, nn.n0.z, nn.n0.w, nn.n2.x, nn.n2.y, o.w, h.t, &tn0);

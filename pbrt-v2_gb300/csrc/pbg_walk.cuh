@@ -105,6 +105,22 @@ __device__ __forceinline__ bool slab(const RayFma& r, float lx, float hx, float 
     return tn <= fmaf(fabsf(tf), kSlabWiden, tf);
 }
 
+// A node in two 32-byte loads (sm_100 and later; nodes start on multiples of
+// their 64 bytes) instead of four of 16: the ordered walk of 921,600 rays 642
+// -> 635 us, direct lighting's packets 870 -> 867 us a frame.
+__device__ __forceinline__ BvhNode load_node(const BvhNode* p) {
+    BvhNode n;
+    float4 a;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(n.n0.x), "=f"(n.n0.y), "=f"(n.n0.z), "=f"(n.n0.w), "=f"(n.n1.x), "=f"(n.n1.y), "=f"(n.n1.z), "=f"(n.n1.w)
+        : "l"(p));
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(n.n2.x), "=f"(n.n2.y), "=f"(n.n2.z), "=f"(n.n2.w), "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+        : "l"(reinterpret_cast<const char*>(p) + 32));
+    n.n3 = make_int4(__float_as_int(a.x), __float_as_int(a.y), __float_as_int(a.z), __float_as_int(a.w));
+    return n;
+}
+
 // The walk's stack.  PACK: one 8-byte entry (one local load per pop) when
 // the scene allows it: a child reference, with a leaf's record start (below
 // 2^24) and triangle count (below 128) packed into one negative word, and
