@@ -504,7 +504,10 @@ int finalize_keys(pbg_scene* s, const int32_t* pos, const float4* o, const float
 
 // The group range is cut so that about tune.naive_ctas CTAs per SM (16 unless
 // tuned: 181 / 170 / 181 us for 8 / 16 / 32 at the sizes above, 256-thread
-// CTAs 191 / 210 / 240) run; a split has at least four groups.
+// CTAs 191 / 210 / 240) run; a split may be one group, since in a small batch
+// the warps run their groups one after another on an idle chip (1,200 rays and
+// as many shadow rays on 4,000 triangles: 72 us with at least four, 48 so; all
+// pairs: 62).
 static void naive_launch_shape(pbg_scene* s, int64_t n, int32_t* ngroups, int32_t* per_split, unsigned* splits) {
     const int64_t ray_ctas = (n + kNaiveThreads - 1) / kNaiveThreads;
     int sms = 152;
@@ -514,7 +517,7 @@ static void naive_launch_shape(pbg_scene* s, int64_t n, int32_t* ngroups, int32_
     // the triangles that every ray tests count as groups of their own here
     const int64_t units = ng + (s->unculled + kNaiveGroup - 1) / kNaiveGroup;
     int64_t want = (per_sm * (int64_t)sms + ray_ctas - 1) / ray_ctas;
-    want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, (units + 3) / 4), 65535));
+    want = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, units), 65535));
     *ngroups = (int32_t)ng;
     *per_split = (int32_t)((ng + want - 1) / want);
     *splits = (unsigned)want;
