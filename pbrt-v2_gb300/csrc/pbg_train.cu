@@ -93,10 +93,25 @@ __device__ __forceinline__ void stage_tile(uint8_t* dst, const uint16_t* src) {
 }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Programmatic dependent launch: this grid's successor may start once every
-// CTA has come here; this grid's predecessor is complete, its writes visible.
-__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launch: once the predecessor is complete and its
+// writes are visible, this grid's successor may start (as soon as every CTA
+// has come here).  In this order no more than one grid waits beside the one
+// that works; released before its own wait, a grid of a later step could
+// start, and its SM's L1 fill with an earlier step's lines, while the step
+// between them was still to write them.
+__device__ __forceinline__ void grid_dependency_wait_and_release() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// What a grid that this one overlaps has written: from L2, and not before the
+// wait above (volatile, no const __restrict__ on the pointer, so neither the
+// compiler nor an L1 line from before the wait can answer it).
+__device__ __forceinline__ float load_written(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // A tile [rows x cols] used with its columns along K (as stored) or with its
 // rows along K (transposed: MN-major), from K step ks (16 elements of K each).
@@ -111,8 +126,7 @@ constexpr uint32_t kAT = 1u << 15, kBT = 1u << 16;  // instruction descriptor: A
 
 __global__ void __launch_bounds__(kTrainThreads, 1)
     train_kernel(const uint16_t* __restrict__ X, const int32_t* __restrict__ label, int tiles,
-                 const uint16_t* __restrict__ Wb, const float* __restrict__ P, float scale,
-                 float* __restrict__ part, int* status) {
+                 const uint16_t* Wb, const float* P, float scale, float* part, int* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sX = smem;
     uint8_t* sW1 = sX + kTX;
@@ -147,18 +161,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     // launch): what does not depend on it goes first -- the first tile's
     // features, barriers, tensor memory -- then the wait, then the weights.
     stage_tile<kTile, kFeat, kXCols>(sX, X + (size_t)blockIdx.x * kTile * kFeat);
-    grid_dependents_launch();
-    grid_dependency_wait();
+    grid_dependency_wait_and_release();
     stage_tile<kHidden, kFeat, kFeat>(sW1, Wb + kOffW1);
     stage_tile<kHidden, kHidden, kHidden>(sW2, Wb + kOffW2);
     stage_tile<kClusters, kHidden, kHidden>(sW3, Wb + kOffW3);
     if (threadIdx.x < kTile * 2)  // the padding columns of X stay zero
         *(uint4*)(sX + core_offset(threadIdx.x >> 1, kFeat + 8 * (threadIdx.x & 1), kXCols)) = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < kHidden) {
-        sb1[threadIdx.x] = P[kOffB1 + threadIdx.x];
-        sb2[threadIdx.x] = P[kOffB2 + threadIdx.x];
+        sb1[threadIdx.x] = load_written(P + kOffB1 + threadIdx.x);
+        sb2[threadIdx.x] = load_written(P + kOffB2 + threadIdx.x);
     }
-    if (threadIdx.x < kClusters) sb3[threadIdx.x] = P[kOffB3 + threadIdx.x];
+    if (threadIdx.x < kClusters) sb3[threadIdx.x] = load_written(P + kOffB3 + threadIdx.x);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -404,25 +417,23 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 // Sums the partial gradients in CTA order, then either stores them (grads)
 // or takes the SGD step with momentum on the FP32 parameters and refreshes
 // the BF16 weights.  W1's columns past the 105 features are padding: never
-// updated, zero in BF16.  Four partials in flight per thread hide the L2
+// updated, zero in BF16.  Eight partials in flight per thread hide the L2
 // latency of the 64 that 8,192 records leave.
 __global__ void __launch_bounds__(256)
-    apply_kernel(const float* __restrict__ part, int nparts, float* __restrict__ P, float* __restrict__ V,
-                 uint16_t* __restrict__ Wb, float* __restrict__ grads, float* __restrict__ acc, float lr, float mom) {
+    apply_kernel(const float* part, int nparts, float* P, float* V, uint16_t* Wb, float* grads, float* acc, float lr, float mom) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    grid_dependents_launch();
-    grid_dependency_wait();
+    grid_dependency_wait_and_release();
     if (i >= kParams + 2) return;
     float s = 0.f;
     int k = 0;
     for (; k + 8 <= nparts; k += 8) {
         float t[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t[j] = part[(size_t)(k + j) * kPartFloats + i];
+        for (int j = 0; j < 8; ++j) t[j] = load_written(part + (size_t)(k + j) * kPartFloats + i);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += t[j];
     }
-    for (; k < nparts; ++k) s += part[(size_t)k * kPartFloats + i];
+    for (; k < nparts; ++k) s += load_written(part + (size_t)k * kPartFloats + i);
     if (i >= kParams) {
         acc[i - kParams] = s;
         return;
@@ -435,9 +446,9 @@ __global__ void __launch_bounds__(256)
         Wb[i] = 0;
         return;
     }
-    const float v = mom * V[i] + s;
+    const float v = mom * load_written(V + i) + s;
     V[i] = v;
-    const float w = P[i] - lr * v;
+    const float w = load_written(P + i) - lr * v;
     P[i] = w;
     Wb[i] = f2bf(w);
 }
