@@ -486,6 +486,12 @@ static const void* device_view(int device, const void* p) {
     return (device >= 0 && device < 64 && ats[device].load() == 2) ? p : nullptr;
 }
 
+// The same for an array of 4-byte words that a kernel reads or writes one by
+// one: nullptr off a word boundary, where copies still work.
+static const void* device_words(int device, const void* p) {
+    return ((uintptr_t)p & 3u) == 0 ? device_view(device, p) : nullptr;
+}
+
 // Caller SoA rows read in place (device-usable addresses) -> 16-byte records,
 // the validity mask copied alongside.
 __global__ void pack_rows_kernel(const float* __restrict__ ox, const float* __restrict__ oy,
@@ -579,7 +585,7 @@ static int stage_rays(pbg_scene* s, const pbg_rays* r, int64_t n, float4** o, fl
         const float* rows[8] = {r->ox, r->oy, r->oz, r->dx, r->dy, r->dz, r->mint, r->maxt};
         const float* dv[8];
         bool direct = true;
-        for (int k = 0; k < 8 && direct; ++k) direct = (dv[k] = (const float*)device_view(s->device, rows[k]));
+        for (int k = 0; k < 8 && direct; ++k) direct = (dv[k] = (const float*)device_words(s->device, rows[k]));
         const uint8_t* vin = nullptr;
         if (direct && r->valid) direct = (vin = (const uint8_t*)device_view(s->device, r->valid)) != nullptr;
         if (direct) {
@@ -771,7 +777,7 @@ static int occluded_in_parts(pbg_scene* s, const pbg_rays* r, int64_t n, uint8_t
     const float* rows[8] = {r->ox, r->oy, r->oz, r->dx, r->dy, r->dz, r->mint, r->maxt};
     const float* dv[8];
     for (int k = 0; k < 8; ++k)
-        if (!(dv[k] = (const float*)device_view(s->device, rows[k]))) return PBG_OK;
+        if (!(dv[k] = (const float*)device_words(s->device, rows[k]))) return PBG_OK;
     const uint8_t* vin = nullptr;
     if (r->valid && !(vin = (const uint8_t*)device_view(s->device, r->valid))) return PBG_OK;
     uint8_t* po = (uint8_t*)device_view(s->device, occ);
@@ -1306,10 +1312,10 @@ int pbg_intersect(pbg_scene* s, const pbg_rays* r, int64_t n, pbg_hits* out) {
     rc = run_nearest(s, o, d, valid, n, (int32_t*)w.prim.ptr, (float*)w.t.ptr, (float*)w.b1.ptr,
                      (float*)w.b2.ptr, s->stream);
     if (rc) return rc;
-    int32_t* pp = (int32_t*)device_view(s->device, out->prim);
-    float* pt = (float*)device_view(s->device, out->t);
-    float* p1 = (float*)device_view(s->device, out->b1);
-    float* p2 = (float*)device_view(s->device, out->b2);
+    int32_t* pp = (int32_t*)device_words(s->device, out->prim);
+    float* pt = (float*)device_words(s->device, out->t);
+    float* p1 = (float*)device_words(s->device, out->b1);
+    float* p2 = (float*)device_words(s->device, out->b2);
     if (pp && pt && p1 && p2) {
         store_hits_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
             (const int32_t*)w.prim.ptr, (const float*)w.t.ptr, (const float*)w.b1.ptr,
@@ -1396,10 +1402,10 @@ int pbg_hit_geometry(pbg_scene* s, const pbg_rays* r, const pbg_hits* h, int64_t
     // The hits are read in place where the GPU can address them (640 x 640
     // hits: 390 us by copies, 332 so); the results, in pages that are often
     // new, go back by the copy engine (a kernel's stores: 494 us).
-    const int32_t* prim = (const int32_t*)device_view(s->device, h->prim);
-    const float* t = (const float*)device_view(s->device, h->t);
-    const float* b1 = (const float*)device_view(s->device, h->b1);
-    const float* b2 = (const float*)device_view(s->device, h->b2);
+    const int32_t* prim = (const int32_t*)device_words(s->device, h->prim);
+    const float* t = (const float*)device_words(s->device, h->t);
+    const float* b1 = (const float*)device_words(s->device, h->b1);
+    const float* b2 = (const float*)device_words(s->device, h->b2);
     if (!prim || !t || !b1 || !b2) {
         PBG_CUDA(cudaMemcpyAsync(w.prim.ptr, h->prim, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
         PBG_CUDA(cudaMemcpyAsync(w.t.ptr, h->t, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream));
