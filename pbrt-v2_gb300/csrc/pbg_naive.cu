@@ -369,17 +369,18 @@ __global__ void __launch_bounds__(kNaiveThreads)
         }
     };
 
-    // the triangles that every ray tests, shared out over the splits
+    // the triangles that every ray tests, shared out over the splits; a warp
+    // leaves once its rays are occluded, or if none of them is valid
     const int32_t u0 = (int32_t)((int64_t)unculled * blockIdx.y / gridDim.y);
     const int32_t u1 = (int32_t)((int64_t)unculled * (blockIdx.y + 1) / gridDim.y);
     for (int32_t j = u0; j < u1; j += kNaiveGroup) {
-        if (ANY && __all_sync(full, done)) break;
+        if (__all_sync(full, done)) break;
         load(j, min(kNaiveGroup, u1 - j));
         test_all(min(kNaiveGroup, u1 - j));
     }
     const int32_t g0 = min((int32_t)blockIdx.y * per_split, ngroups), g1 = min(g0 + per_split, ngroups);
     for (int32_t g = g0; g < g1; ++g) {
-        if (ANY && __all_sync(full, done)) break;
+        if (__all_sync(full, done)) break;
         const int32_t first = unculled + g * kNaiveGroup;
         const int32_t cnt = min(kNaiveGroup, ntri - first);
         unsigned meet = full, side = 0;  // lanes whose rays test every member; members that the others test too
