@@ -1203,12 +1203,12 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
                         qb = tq;
                         nl += 2;
                     }
-                    const auto kernel = stats ? rh_split_test_kernel<ANY, true, false>
-                                        : few ? rh_split_test_kernel<ANY, false, true>
-                                                                        : rh_split_test_kernel<ANY, false, false>;
-                    kernel<<<(unsigned)(sms * kSplitBlocks), 32 * kSplitWarps, 0, st>>>(tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1],
-                                                  nodes + lv.off[0], lv.cnt[0], qa, cnt_of[1], cap, counts + kNextPair, so, sd, keys, mask,
-                                                  leaf_reach, parent_reach, status, stats ? wc : nullptr);
+                    const auto kernel = few ? (stats ? rh_split_test_kernel<ANY, true, true> : rh_split_test_kernel<ANY, false, true>)
+                                            : (stats ? rh_split_test_kernel<ANY, true, false> : rh_split_test_kernel<ANY, false, false>);
+                    kernel<<<(unsigned)(sms * kSplitBlocks), 32 * kSplitWarps, 0, st>>>(
+                        tsph, (const TriRec*)s->tris.ptr, t0, t1, nodes + lv.off[1], nodes + lv.off[0], lv.cnt[0], qa,
+                        cnt_of[1], cap, counts + kNextPair, so, sd, keys, mask, leaf_reach, parent_reach, status,
+                        stats ? wc : nullptr);
                     fused = true;
                     ++nl;
                     break;

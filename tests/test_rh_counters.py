@@ -1,0 +1,32 @@
+"""rayhierarchy's work counters (profiling level 2) describe the form of the
+leaf tests that runs without them: a small batch's warps take one leaf of a
+(cluster, parent) pair each and test the members against the parent again."""
+import numpy as np
+import pytest
+
+import pbg_import
+
+pbg_import.load()
+from pbrt_gb300 import accel as A  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def test_small_batch_counts(gpu_lib):
+    g = np.random.default_rng(4)
+    turn = g.uniform(0, 7, (32, 1)) + np.arange(3) * 2 * np.pi / 3  # one cluster of equal triangles about the origin
+    tris = np.stack([0.3 * np.cos(turn), 0.3 * np.sin(turn), np.zeros((32, 3))], -1) + g.uniform(-0.01, 0.01, (32, 1, 3))
+    tris = tris.astype(np.float32).reshape(32, 9)
+    leaves, parents, fan = 5, 2, 4
+    rays = np.zeros((8, 32 * leaves), np.float32)  # one eye, into the cluster: every node reaches every member
+    rays[2] = -5.0
+    rays[3:5] = g.uniform(-0.02, 0.02, (2, 32 * leaves))
+    rays[5], rays[7] = 1.0, np.inf
+    acc = A.MakeAccelerator("rayhierarchy", tris)
+    acc.profile(2)
+    acc.IntersectP(rays)
+    work = acc.stats()["work"]
+    acc.close()
+    # the seed's pairs; each pair's members against the parent, once per leaf; the members against the leaves
+    assert work["node_tests"] == parents + parents * fan * 32 + leaves * 32
+    assert work["leaves"] == leaves
