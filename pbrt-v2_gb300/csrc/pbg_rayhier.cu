@@ -84,9 +84,9 @@ __device__ __forceinline__ float beam_spread(float c, bool plain) {
 
 // A batch of at most this many rays has launches and few long pairs to wait
 // for: its leaf build zeroes the traversal's words, its finalize kernel
-// publishes the status, its split tests take a leaf per warp and its other
-// kernels fewer CTAs; larger batches use memsets, a kernel of its own and a
-// pair per warp.  Frames of 131,400 / 256,000 / 700,000 rays: 452 / 618 /
+// publishes the status, its split tests take a leaf per warp while there are
+// few pairs, and its other kernels fewer CTAs; larger batches use memsets, a
+// kernel of its own and a pair per warp.  Frames of 131,400 / 256,000 / 700,000 rays: 452 / 618 /
 // 1,664 us in the first form, 469 / 624 / 1,439 in the second.
 constexpr int64_t kFewRays = 1 << 19;
 constexpr int kFewGrid = 12;  // CTAs per SM of their level kernels (of 4, 12, 32: 175, 172, 177 us at 19,159 rays)
@@ -546,11 +546,17 @@ __device__ __forceinline__ uint32_t next_task(unsigned long long* s_lot, uint32_
     return first;
 }
 
-// SMALL (batches of at most kFewRays rays): a warp takes one leaf of a pair
-// and tests the members against the parent again, since with few pairs to a
-// warp the longest one is the kernel's time (a frame of 19,159 rays 228 us ->
-// 198).
-template <bool ANY, bool STATS, bool SMALL>
+// FEW (batches of at most kFewRays rays): with less than kByLeaf pairs to a
+// warp, where the longest one is the kernel's time, a warp takes one leaf of a
+// pair and tests the members against the parent again (19,159 camera and
+// shadow rays on 12,000 triangles: 163 us, 194 by pairs).  With more of them
+// that only adds work, and the parents' live bounds, which one leaf cannot
+// lower, cull nothing: 19,159 bounce rays on 1,000,000 triangles 22.2 ms by
+// leaves, 17.9 by pairs; 518,400 camera rays there 900 us, 588.  Lines at 0.3,
+// 1, 4 and 12 pairs to a warp: 192 / 167 / 163 / 166 us for the first, 312 /
+// 315 / 313 / 331 for 19,159 camera and shadow rays on 181,250 triangles.
+constexpr uint32_t kByLeaf = 4;
+template <bool ANY, bool STATS, bool FEW>
 __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
     rh_split_test_kernel(const float4* __restrict__ spheres, const TriRec* __restrict__ tris, int32_t t0,
                          int32_t t1, const RayNode* __restrict__ level1, const RayNode* __restrict__ leaves,
@@ -569,7 +575,8 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
     const uint32_t nin = min(*in_count, cap);
     const int lane = threadIdx.x & 31;
     WorkCount c_;
-    const int64_t ntask = SMALL ? (int64_t)nin * kFan : nin;
+    const bool by_leaf = FEW && nin < kByLeaf * kSplitWarps * gridDim.x;
+    const int64_t ntask = by_leaf ? (int64_t)nin * kFan : nin;
     const uint32_t deal = ntask >= (int64_t)(kDeal * kSplitWarps) * gridDim.x ? kDeal : 1u;
     if (threadIdx.x == 0) s_lot = deal;
     __syncthreads();
@@ -578,7 +585,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
         if (lane == 0) task = next_task(&s_lot, next, deal);
         task = __shfl_sync(full, task, 0);
         if (task >= ntask) break;
-        const Pair pr = in[SMALL ? task / kFan : task];
+        const Pair pr = in[by_leaf ? task / kFan : task];
         const int64_t t = (int64_t)pr.tri * kClusterTris + lane;
         bool pass = false;
         float4 sph = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -607,9 +614,9 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
         }
         __syncwarp();
         // Every eight of them against the kFan leaves at once: lane = (member,
-        // leaf).  SMALL: all against the task's leaf, lane = member.
+        // leaf).  by_leaf: all against the task's leaf, lane = member.
         const int64_t first = (int64_t)pr.node * kFan;
-        const int mine = SMALL ? (int)(task % kFan) : lane % kFan;
+        const int mine = by_leaf ? (int)(task % kFan) : lane % kFan;
         const int64_t my_leaf = first + mine;
         RayNode nd;
         nd.c = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -618,8 +625,8 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
         if (!ANY && rays) nd.c.y = fminf(nd.c.y, live_reach(leaf_reach + my_leaf));
         unsigned mine_reached = 0;  // lane k: the leaves that member k reaches, one bit each
 #pragma unroll 1
-        for (int k0 = 0; k0 < np; k0 += SMALL ? 32 : 32 / kFan) {
-            const int k = k0 + (SMALL ? lane : lane / kFan);
+        for (int k0 = 0; k0 < np; k0 += by_leaf ? 32 : 32 / kFan) {
+            const int k = k0 + (by_leaf ? lane : lane / kFan);
             bool reach = false;
             if (k < np && rays) {
                 if (STATS) c_.node++;
@@ -633,17 +640,17 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
                 }
             }
             const unsigned b = __ballot_sync(full, reach);
-            if (SMALL)
+            if (by_leaf)
                 mine_reached = reach ? 1u << mine : 0u;
             else if (lane / (32 / kFan) == k0 / (32 / kFan))
                 mine_reached = b >> (lane % (32 / kFan) * kFan) & ((1u << kFan) - 1u);
         }
         float parent_new = 0.f;  // max of the leaves' bounds after this pair
 #pragma unroll 1
-        for (int c = SMALL ? mine : 0, c1 = SMALL ? c + 1 : kFan; c < c1; ++c) {
+        for (int c = by_leaf ? mine : 0, c1 = by_leaf ? c + 1 : kFan; c < c1; ++c) {
             const int64_t leaf = first + c;
             unsigned m = __ballot_sync(full, mine_reached >> c & 1u);
-            const float leaf_now = __shfl_sync(full, nd.c.y, c);  // SMALL: every lane's leaf
+            const float leaf_now = __shfl_sync(full, nd.c.y, c);  // by_leaf: every lane's leaf
             const int count = __shfl_sync(full, __float_as_int(nd.c.z), c);
             if (!m) {
                 if (!ANY && count > 0) parent_new = fmaxf(parent_new, leaf_now);
@@ -743,7 +750,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps, kSplitBlocks)
                 parent_new = fmaxf(parent_new, fminf(b, leaf_now));
             }
         }
-        if (!ANY && !SMALL && lane == 0 && parent_new < parent_now) lower_reach(parent_reach + pr.node, parent_new);
+        if (!ANY && !by_leaf && lane == 0 && parent_new < parent_now) lower_reach(parent_reach + pr.node, parent_new);
     }
     if (STATS) c_.flush(wc);
 }

@@ -30,3 +30,20 @@ def test_small_batch_counts(gpu_lib):
     # the seed's pairs; each pair's members against the parent, once per leaf; the members against the leaves
     assert work["node_tests"] == parents + parents * fan * 32 + leaves * 32
     assert work["leaves"] == leaves
+
+
+def test_many_pairs_count_as_a_large_batch(gpu_lib):
+    """By leaves only while there are few pairs to a warp: incoherent rays on
+    either side of the small batches' line do the same work (by leaves each
+    member is tested against the parent four times)."""
+    from pbrt_gb300 import scenes as S
+    line = 1 << 19
+    acc = A.MakeAccelerator("rayhierarchy", S.terrain_icospheres(seed=2, grid=20, n_spheres=2)["tris"])
+    rays = S.random_rays(line + 32, -6.0, 6.0, seed=8)
+    tests = []
+    for n in (line, line + 32):
+        acc.profile(2)
+        acc.Intersect(np.ascontiguousarray(rays[:, :n]))
+        tests.append(acc.stats()["work"]["node_tests"])
+    acc.close()
+    assert tests[0] <= 1.1 * tests[1]
