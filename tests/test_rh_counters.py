@@ -47,3 +47,24 @@ def test_many_pairs_count_as_a_large_batch(gpu_lib):
         tests.append(acc.stats()["work"]["node_tests"])
     acc.close()
     assert tests[0] <= 1.1 * tests[1]
+
+
+@pytest.mark.parametrize("spread", [0.02, 0.2, 0.3, 3.0])
+@pytest.mark.parametrize("n", [33, 4099, (1 << 19) + 7])
+def test_leaves_about_the_narrow_line(gpu_lib, spread, n):
+    """Nearest hits of leaves whose cones lie on either side of the line where
+    the beam test and the held exact tests stop, as the naive accelerator's."""
+    from pbrt_gb300 import scenes as S
+    tris = S.terrain_icospheres(seed=2, grid=20, n_spheres=2)["tris"]
+    g = np.random.default_rng(n)
+    rays = np.zeros((8, n), np.float32)
+    rays[0:3] = g.uniform(-0.1, 0.1, (3, n)) + np.array([[0.5], [4.0], [-1.0]])
+    rays[3:6] = g.normal(size=(3, n)) * spread + np.array([[0.1], [-1.0], [0.05]])
+    rays[7] = np.where(g.random(n) < 0.2, 4.0, np.inf)
+    ref, acc = A.MakeAccelerator("naive", tris), A.MakeAccelerator("rayhierarchy", tris)
+    want = ref.Intersect(rays.copy())
+    for a, b in zip(acc.Intersect(rays.copy()), want):
+        np.testing.assert_array_equal(a, b)
+    assert (want[0] >= 0).any()
+    acc.close()
+    ref.close()
