@@ -327,9 +327,10 @@ __device__ __forceinline__ bool node_hits_sphere(const RayNode& nd, float4 sph) 
 // So the triangle is missed where the divisor's sign is certain and b1 < 0,
 // b2 < 0 or b1 + b2 > 1 for all of them.  2^-17 of the lengths covers pbrt's
 // rounding of each product (9.1 u with u = 2^-24, see pbg_exact.cuh), the
-// rounding here and that of b1, b2 and their sum; edges, distances and
-// directions of extreme size, where products may overflow or underflow, are
-// never missed, and a NaN anywhere keeps the triangle.
+// rounding here and that of b1, b2 and their sum; edges, distances (a tiny one
+// too: the origins at a vertex) and directions of extreme size, where products
+// may overflow or underflow, are never missed, and a NaN anywhere keeps the
+// triangle.
 __device__ __forceinline__ float rough_len(float x, float y, float z) {
     const float l2 = x * x + y * y + z * z;
     return l2 * rsqrtf(l2);  // within 2^-20, inside the spread's own margin
@@ -354,7 +355,7 @@ __device__ __forceinline__ bool beam_misses(const RayNode& nd, const TriRec& tr)
     const float div = ax * mx + ay * my + az * mz;
     const float n1 = flip_sign(ax * q1x + ay * q1y + az * q1z, div), n2 = flip_sign(ax * q2x + ay * q2y + az * q2z, div);
     const float D = fabsf(div), ee = kTol * ne1 * ne2, rt = fmaf(kTol, nw, r);
-    const bool certain = D > fmaf(spread, rough_len(mx, my, mz), ee) && fminf(ne1, ne2) >= 1.f / kBig &&
+    const bool certain = D > fmaf(spread, rough_len(mx, my, mz), ee) && fminf(fminf(ne1, ne2), nw) >= 1.f / kBig &&
                          fmaxf(fmaxf(ne1, ne2), nw) <= kBig;
     const float n3 = ne1 + ne2;
     return certain && (n1 < -fmaf(spread, rough_len(q1x, q1y, q1z), ne2 * rt) ||
