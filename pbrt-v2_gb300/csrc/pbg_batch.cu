@@ -120,13 +120,13 @@ __global__ void __launch_bounds__(kBatchMaxThreads) batch_trace_kernel(BatchArgs
             WorkCount wc;
             if (any) {
                 const float4 o = a.o4s[r], d = a.d4s[r];
-                WalkHit h{d.w, 0.f, 0.f, -1};
+                WalkHit h = unhit(d);
                 ok &= bvh_walk<true, false, false>(sd.nodes, sd.tris, sd.unculled, o, d, INT32_MIN, 0,
                                                    h, wc);
                 a.occ[r] = h.prim >= 0 ? 1 : 0;
             } else {
                 const float4 o = a.o4n[r], d = a.d4n[r];
-                WalkHit h{d.w, 0.f, 0.f, -1};
+                WalkHit h = unhit(d);
                 ok &= bvh_walk<false, false, false>(sd.nodes, sd.tris, sd.unculled, o, d, INT32_MIN, 0,
                                                     h, wc);
                 const bool hit = h.prim >= 0;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) batch_persistent_kernel(Batc
                     d = any ? a.d4s[r] : a.d4n[r];
                     nd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
                     ri = RayInv{o.x, o.y, o.z, safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)};
-                    h = WalkHit{d.w, 0.f, 0.f, -1};
+                    h = unhit(d);
                     sp = 0;
                     node = 0;
                     ok = true;

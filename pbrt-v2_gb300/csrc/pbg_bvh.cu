@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kBvhThreads, kBvhMinBlocks)
     }
     WorkCount wc;
     const float4 o = ro[ray], d = rd[ray];
-    WalkHit h{d.w, 0.f, 0.f, -1};
+    WalkHit h = unhit(d);
     int32_t fref = INT32_MIN, fcnt = 0;
     if (ORDERED) {
         const int c = pred[ray];
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kPacketThreads)
         }
         const float ndd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
         const RayFma ri = ray_fma(o, d);  // direct lighting's camera rays 308 -> 301 us; the persistent walk is no faster for it
-        WalkHit h{d.w, 0.f, 0.f, -1};
+        WalkHit h = unhit(d);
         bool done = !active;
         if (!done && unculled > 0) done = test_run<ANY, STATS>(tris, 0, unculled, o, d, ndd, h, wc);
         int sp = 0;  // warp-uniform
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
                         d = rd[ray];
                         nd = fabsf(d.x) + fabsf(d.y) + fabsf(d.z);
                         ri = RayInv{o.x, o.y, o.z, safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)};
-                        h = WalkHit{d.w, 0.f, 0.f, -1};
+                        h = unhit(d);
                         sp = 0;
                         node = 0;
                         ok = true;

@@ -171,6 +171,11 @@ struct WalkHit {
     int32_t prim;
 };
 
+// A ray's state before its first hit.  A maxt that is NaN rejects nothing in
+// pbrt's test, as +inf does; a walk's own comparisons with it would reject all
+// that waits on the stack.
+__device__ __forceinline__ WalkHit unhit(float4 d) { return WalkHit{fminf(d.w, INFINITY), 0.f, 0.f, -1}; }
+
 // The exact test of record `rec` and its effect on the hit; returns true when
 // an any-hit query is done.
 template <bool ANY, bool STATS>

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                         rf = ray_fma(o, d);
                         oct = (__float_as_uint(rf.ix) >> 31) | (__float_as_uint(rf.iy) >> 31) << 1 |
                               (__float_as_uint(rf.iz) >> 31) << 2;
-                        h = WalkHit{d.w, 0.f, 0.f, -1};
+                        h = unhit(d);
                         sp = 0;
                         ok = true;
                         gbase = 0;  // the root: slot 0 of a group whose only inner child is node 0
