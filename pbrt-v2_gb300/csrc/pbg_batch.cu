@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kBatchMaxThreads) batch_persistent_kernel(Batc
         while (sp > 0) {
             --sp;
             int32_t ref, cnt;
-            if (stk.get(sp, &ref, &cnt) <= h.t) {
+            if (!(stk.get(sp, &ref, &cnt) > h.t)) {
                 if (cnt == 0) {
                     node = ref;
                 } else {

@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
             --sp;
             int32_t ref, cnt;
             const float te = stk.get(sp, &ref, &cnt);
-            if (te <= h.t) {
+            if (!(te > h.t)) {
                 if (cnt == 0) {
                     node = ref;
                 } else {
@@ -390,12 +390,12 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks)
             if (STATS) wc.leaf++;
             bool done = test_run<ANY, STATS>(tris, leaf_start, leaf_cnt, o, d, nd, h, wc);
             leaf_cnt = 0;
-            if (!done && leafb_cnt > 0 && leafb_t <= h.t) {
+            if (!done && leafb_cnt > 0 && !(leafb_t > h.t)) {
                 if (STATS) wc.leaf++;
                 done = test_run<ANY, STATS>(tris, leafb_start, leafb_cnt, o, d, nd, h, wc);
             }
             leafb_cnt = 0;
-            if (!done && leafc_cnt > 0 && leafc_t <= h.t) {
+            if (!done && leafc_cnt > 0 && !(leafc_t > h.t)) {
                 if (STATS) wc.leaf++;
                 done = test_run<ANY, STATS>(tris, leafc_start, leafc_cnt, o, d, nd, h, wc);
             }

@@ -173,7 +173,8 @@ struct WalkHit {
 
 // A ray's state before its first hit.  A maxt that is NaN rejects nothing in
 // pbrt's test, as +inf does; a walk's own comparisons with it would reject all
-// that waits on the stack.
+// that waits on the stack.  A hit's t may be NaN as well, where products over-
+// or underflow: the walks keep what is not beyond it, !(te > h.t).
 __device__ __forceinline__ WalkHit unhit(float4 d) { return WalkHit{fminf(d.w, INFINITY), 0.f, 0.f, -1}; }
 
 // The exact test of record `rec` and its effect on the hit; returns true when
@@ -288,7 +289,7 @@ __device__ __forceinline__ bool bvh_walk(const BvhNode* __restrict__ nodes, cons
         while (sp > 0) {
             --sp;
             const int2 e = stack[sp];
-            if (__int_as_float(e.y) <= h.t) {
+            if (!(__int_as_float(e.y) > h.t)) {
                 node = e.x;
                 found = true;
                 break;

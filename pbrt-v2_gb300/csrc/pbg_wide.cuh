@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
                     --sp;
                     const int2 e = stack[sp];
                     const float te = __uint_as_float((uint32_t)e.y & 0xffff0000u);
-                    if (te <= h.t) {
+                    if (!(te > h.t)) {
                         gbase = e.x;
                         ghits = (uint32_t)e.y & 0xffu;
                         gimask = ((uint32_t)e.y >> 8) & 0xffu;

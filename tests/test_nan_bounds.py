@@ -52,3 +52,27 @@ def test_nan_bounds_in_a_set(gpu_lib, oracle, walk):
         for a, b in zip((prim, t, b1, b2), want):
             np.testing.assert_array_equal(a.cpu().numpy()[part], b)
         np.testing.assert_array_equal(occ.cpu().numpy()[part] != 0, oracle.anyhit(tris, r) != 0)
+
+
+@pytest.mark.parametrize("walk", [0, 1, 2, 3, 4, 5, 6])
+def test_walk_goes_on_behind_a_nan_hit(gpu_lib, oracle, walk):
+    """A triangle so small that its divisor is subnormal is hit at a distance
+    that is NaN, after which pbrt accepts whatever it hits: what lies behind,
+    of higher indices, is found by every walk."""
+    tiny = np.array([[0, 0, 0, 1e-15, 0, 0, 0, 1e-27, 0]], np.float32)
+    g = np.random.default_rng(1)
+    a = g.uniform(-3, 3, (400, 2))
+    behind = np.zeros((400, 3, 3))
+    behind[:, :, 2] = g.uniform(1, 9, (400, 1))
+    behind[:, :, :2] = a[:, None] * 0.02 + np.array([[-1, -1], [1.5, -1], [-1, 1.5]]) * g.uniform(0.02, 4, (400, 1, 1))
+    tris = np.concatenate([tiny, behind.reshape(400, 9).astype(np.float32)])
+    rays = np.zeros((8, 40), np.float32)
+    rays[2], rays[5], rays[7] = -1e-5, 1.0, np.inf
+    want = oracle.nearest(tris, rays.copy())
+    assert np.isnan(oracle.nearest(tiny, rays.copy())[1]).all() and (want[0] > 0).all()
+    acc = A.MakeAccelerator("ray-bvh", tris, {"walk": walk})
+    for _ in range(2):
+        for a, b in zip(acc.Intersect(rays.copy()), want):
+            np.testing.assert_array_equal(a, b)
+        assert (acc.IntersectP(rays) == ord("1")).all()
+    acc.close()
