@@ -485,7 +485,8 @@ int pbg_tc_gemm_bf16(const uint16_t* A, const uint16_t* B, float* C, int32_t M, 
  * o4/d4 (16-byte ray records, valid may be NULL) with every candidate shape
  * of the scene's accelerator -- naive: CTAs per SM of the triangle splits
  * (2, 4, 8, 16); rayhierarchy: nodes of the seed level (64, 256, 1024) x
- * CTAs per SM of the grid-stride kernels (16, 32), per query kind; ray-bvh:
+ * CTAs per SM of the grid-stride kernels (16, 32; 12, 32 for a batch of up to
+ * 2^19 rays, kept for such batches), per query kind; ray-bvh:
  * walk 1-6 (pbg_params.walk) for this batch class -- times each on `stream`
  * (best of `reps` after a warm-up run), checks that every candidate's
  * results equal the first one's bit for bit (else PBG_ERR_INTERNAL and the

@@ -78,9 +78,10 @@ constexpr int kClusterTris = 32;
 struct Tunables {
     int naive_ctas = 16;     // naive: CTAs per SM the triangle splits aim for
     // rayhierarchy [any-hit]: nodes of the level the descent starts at (at
-    // most), CTAs per SM of the grid-stride kernels
+    // most); [any-hit][small batch]: CTAs per SM of the grid-stride kernels
+    // (0: rh_default_grid)
     int rh_seed[2] = {1024, 1024};
-    int rh_grid[2] = {32, 32};
+    int rh_grid[2][2] = {{0, 0}, {0, 0}};
     int bvh_walk[2][2] = {{0, 0}, {0, 0}};  // ray-bvh [any-hit][incoherent]: 0 automatic, else pbg_params.walk's 1-6
 };
 
@@ -195,6 +196,10 @@ int wide_nearest(pbg_scene* s, bool coop, const float4* o, const float4* d, cons
                  cudaStream_t st);
 int wide_occluded(pbg_scene* s, bool coop, const float4* o, const float4* d, const uint8_t* valid,
                   const int32_t* perm, int64_t n, QueueRef q, int32_t* occluders, uint8_t* occ, cudaStream_t st);
+// Whether n rays are a small batch of rayhierarchy, and the CTAs per SM of its
+// grid-stride kernels untuned.
+bool rh_small_batch(int64_t n);
+int rh_default_grid(bool small);
 int rh_nearest(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,
                int32_t* prim, float* t, float* b1, float* b2, cudaStream_t st);
 int rh_occluded(pbg_scene* s, const float4* o, const float4* d, const uint8_t* valid, int64_t n,

@@ -89,7 +89,11 @@ __device__ __forceinline__ float beam_spread(float c, bool plain) {
 // kernel of its own and a pair per warp.  Frames of 131,400 / 256,000 / 700,000 rays: 452 / 618 /
 // 1,664 us in the first form, 469 / 624 / 1,439 in the second.
 constexpr int64_t kFewRays = 1 << 19;
-constexpr int kFewGrid = 12;  // CTAs per SM of their level kernels (of 4, 12, 32: 175, 172, 177 us at 19,159 rays)
+// CTAs per SM of the level kernels where tune.rh_grid has none: 12 for small
+// batches (of 4, 12, 32: 175, 172, 177 us at 19,159 rays), 32 for others (best
+// of 4, 8, 16, 32 on the terrain frame).
+bool rh_small_batch(int64_t n) { return n <= kFewRays; }
+int rh_default_grid(bool small) { return small ? 12 : 32; }
 
 // Words of device memory that a batch starts from zero (its keys or
 // occlusion bits, counters, bounds).
@@ -1076,7 +1080,7 @@ static int rh_build(pbg_scene* s, const float4* o, const float4* d, const uint8_
     const bool keep_o = order == kOrderOrigin && w.origin_reused && had_origins &&
                         before[0] == w.ray_o2.ptr && before[1] == w.nodes.ptr;
     if (s->ntri > 0 && (rc = rh_workspace(s, *lv, order == kOrderOrigin, zero))) return rc;
-    const bool few = n <= kFewRays;
+    const bool few = rh_small_batch(n);
     for (int k = 0; !few && k < zero->count; ++k) PBG_CUDA(cudaMemsetAsync(zero->p[k], 0, (size_t)zero->n[k] * 4, st));
     prof_begin(s, st);
     (few ? leaf_build_kernel<true> : leaf_build_kernel<false>)<<<(unsigned)((nleaf * 32 + 255) / 256), 256, 0, st>>>(
@@ -1148,11 +1152,9 @@ static int rh_traverse(pbg_scene* s, const Levels& lv, const float4* so, const f
     const uint32_t cap = queue_capacity(s);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    // grid-stride kernels: 32 CTAs per SM measured best of 4, 8, 16, 32 on
-    // the terrain frame (tune.rh_grid)
-    const bool few = nleaf * kLeafRays <= kFewRays;
-    const int per_sm = s->tune.rh_grid[ANY] > 0 ? s->tune.rh_grid[ANY] : 32;
-    const unsigned grid = (unsigned)(sms * (few ? std::min(per_sm, kFewGrid) : per_sm));
+    const bool few = rh_small_batch(nleaf * kLeafRays);
+    const int tuned_grid = s->tune.rh_grid[ANY][few];
+    const unsigned grid = (unsigned)(sms * (tuned_grid > 0 ? tuned_grid : rh_default_grid(few)));
     const bool stats = s->prof.level >= 2;
     unsigned long long* wc = (unsigned long long*)s->workc.ptr;
     int* status = (int*)s->err.ptr;

@@ -7,8 +7,9 @@
 // vary without changing any result are tuned per scene on a sample batch:
 //   naive         CTAs per SM that the triangle splits aim for: 2, 4, 8, 16
 //   rayhierarchy  nodes of the level the descent is seeded at (64, 256,
-//                 1024) x CTAs per SM of the grid-stride kernels (16, 32),
-//                 kept apart for nearest-hit and any-hit batches
+//                 1024) x CTAs per SM of the grid-stride kernels (16, 32; 12,
+//                 32 for batches of up to 2^19 rays, whose setting is kept
+//                 apart), kept apart for nearest-hit and any-hit batches
 //   ray-bvh       the walk for this batch class (any-hit or not, coherent
 //                 or not): one thread per ray, persistent warps, warp
 //                 packets over the ray hierarchy's leaves (sorted) or over
@@ -56,31 +57,31 @@ struct Candidate {
     int v[3];
 };
 
-void apply(pbg_scene* s, int any, int incoherent, const Candidate& c) {
+void apply(pbg_scene* s, int any, int incoherent, bool small, const Candidate& c) {
     switch (s->accel) {
         case PBG_ACCEL_NAIVE: s->tune.naive_ctas = c.v[0]; break;
         case PBG_ACCEL_RAYHIERARCHY:
             s->tune.rh_seed[any] = c.v[0];
-            s->tune.rh_grid[any] = c.v[1];
+            s->tune.rh_grid[any][small] = c.v[1];
             break;
         case PBG_ACCEL_RAYBVH: s->tune.bvh_walk[any][incoherent] = c.v[0]; break;
     }
 }
 
-Candidate current(const pbg_scene* s, int any, int incoherent) {
+Candidate current(const pbg_scene* s, int any, int incoherent, bool small) {
     Candidate c{{0, 0, 0}};
     switch (s->accel) {
         case PBG_ACCEL_NAIVE: c.v[0] = s->tune.naive_ctas; break;
         case PBG_ACCEL_RAYHIERARCHY:
             c.v[0] = s->tune.rh_seed[any];
-            c.v[1] = s->tune.rh_grid[any];
+            c.v[1] = s->tune.rh_grid[any][small];
             break;
         case PBG_ACCEL_RAYBVH: c.v[0] = s->tune.bvh_walk[any][incoherent]; break;
     }
     return c;
 }
 
-std::vector<Candidate> candidates(const pbg_scene* s) {
+std::vector<Candidate> candidates(const pbg_scene* s, bool small) {
     std::vector<Candidate> out;
     switch (s->accel) {
         case PBG_ACCEL_NAIVE:
@@ -88,7 +89,7 @@ std::vector<Candidate> candidates(const pbg_scene* s) {
             break;
         case PBG_ACCEL_RAYHIERARCHY:
             for (int seed : {1024, 64, 256})
-                for (int grid : {32, 16}) out.push_back({{seed, grid, 0}});
+                for (int grid : {rh_default_grid(small), small ? 32 : 16}) out.push_back({{seed, grid, 0}});
             break;
         case PBG_ACCEL_RAYBVH:
             if (s->params.walk != 0) {
@@ -123,8 +124,9 @@ extern "C" int pbg_autotune(pbg_scene* s, const float* o4, const float* d4, cons
     cudaStream_t st = stream ? (cudaStream_t)stream : s->stream;
     const int any = query & 1, incoherent = (query >> 1) & 1;
     if (reps < 1) reps = 3;
-    const std::vector<Candidate> cand = candidates(s);
-    const Candidate before = current(s, any, incoherent);
+    const bool small = rh_small_batch(n);
+    const std::vector<Candidate> cand = candidates(s, small);
+    const Candidate before = current(s, any, incoherent, small);
     const int saved_hint = s->walk_hint;
     const float4* o = (const float4*)o4;
     const float4* d = (const float4*)d4;
@@ -135,7 +137,7 @@ extern "C" int pbg_autotune(pbg_scene* s, const float* o4, const float* d4, cons
     int rc = PBG_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto fail = [&](int code) {
-        apply(s, any, incoherent, before);
+        apply(s, any, incoherent, small, before);
         s->walk_hint = saved_hint;
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
@@ -162,7 +164,7 @@ extern "C" int pbg_autotune(pbg_scene* s, const float* o4, const float* d4, cons
     float best_ms = 0.f;
     int best = -1;
     for (int k = 0; k < nc; ++k) {
-        apply(s, any, incoherent, cand[k]);
+        apply(s, any, incoherent, small, cand[k]);
         DeviceBuffer& dst = k == 0 ? ref : cur;
         if ((rc = run(dst))) return fail(rc);  // warm-up (and the compared result)
         float ms = 0.f;
@@ -212,7 +214,7 @@ extern "C" int pbg_autotune(pbg_scene* s, const float* o4, const float* d4, cons
     }
     out->ncandidates = nc;
     out->best = best;
-    apply(s, any, incoherent, cand[best]);
+    apply(s, any, incoherent, small, cand[best]);
     s->walk_hint = saved_hint;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
