@@ -27,6 +27,7 @@
 
 #include "pbg_internal.h"
 #include "pbg_learn.h"
+#include "pbg_quotient.h"
 #include "pbg_tc.cuh"
 
 namespace pbg {
@@ -291,16 +292,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
                       (spart[(8 + j) * kTile + r] + spart[(24 + j) * kTile + r]);
         const float s = ((lsum[0] + lsum[4]) + (lsum[2] + lsum[6])) + ((lsum[1] + lsum[5]) + (lsum[3] + lsum[7]));
         __syncthreads();  // spart's place becomes dZ3
-        // e / s as e * (1 / s) corrected by its remainder (Markstein 1990):
-        // the rounded quotient, s in [1, 256]
         const float inv = 1.f / s;
 #pragma unroll 1
         for (int c = 8 * g; c < kClusters; c += 64) {
             tmem_ld8x2(tl + (uint32_t)c, tl + (uint32_t)c + 32u, v);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                const float q0 = v[j] * inv;
-                v[j] = fmaf(fmaf(-q0, s, v[j]), inv, q0);
+                v[j] = quotient(v[j], s, inv);
                 if (c + column_of(j) == y) {
                     loss -= __logf(fmaxf(v[j], 1e-30f));
                     right += am == y ? 1.f : 0.f;
