@@ -404,8 +404,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             out[kParams + threadIdx.x] = t;
         }
     } else if (threadIdx.x == 0) {
-        // give in-flight MMAs one more bounded window before TMEM is released
-        mbar_wait_bounded(bar, phase, status);
+        // MMAs in flight get one more bounded window before TMEM is released:
+        // those of the wait that failed, then those issued behind it
+        if (mbar_wait_bounded(bar, phase ^ 1u, status)) {
+            tc_commit(bar);
+            mbar_wait_bounded(bar, phase, status);
+        }
     }
     tc_fence_before();
     __syncthreads();
