@@ -52,7 +52,6 @@
 #include "pbg_count.cuh"
 #include "pbg_curve.cuh"
 #include "pbg_internal.h"
-#include "pbg_tma.cuh"
 #include "pbg_walk.cuh"
 
 namespace pbg {

@@ -1,9 +1,6 @@
-// pbg_tma.cuh -- bulk (TMA) copies into shared memory with mbarrier
-// completion, and bounded waits.
+// pbg_tma.cuh -- shared-memory barriers for asynchronous completion (the
+// tensor-core kernels' MMAs), bounded waits on them, device status words.
 //
-// Tiles of triangle records are contiguous in global memory, so the 1-D bulk
-// form cp.async.bulk suffices: source and destination 16-byte aligned, size a
-// multiple of 16 bytes (TriRec is 48 bytes, so every tile qualifies).
 // Every wait is bounded: after kSpinLimit polls it records a status word in
 // global memory and the caller leaves the kernel; no wait can hang the GPU.
 #pragma once
@@ -32,21 +29,6 @@ __device__ __forceinline__ void mbar_fence_init() {
 
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
-                                         uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
