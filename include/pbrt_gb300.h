@@ -76,7 +76,8 @@ typedef struct pbg_params {
                            * chose for the batch class, else 6 for bounce
                            * batches -- nearest hit with a validity mask, and
                            * the renderer's bounces >= 1 --; for the others 4
-                           * nearest-hit from 786,432 rays, 5 any-hit from
+                           * nearest-hit where packets pay (by the rays, the
+                           * triangles and the samples per pixel), 5 any-hit from
                            * 262,144, and 6 below that, or 2 where the scene
                            * has no eight-wide tree yet),
                            * 1 = one thread per ray, 2 = persistent warps refilled
@@ -189,6 +190,10 @@ int pbg_max_rays_per_call(const pbg_scene* scene, int64_t* out);
  * (rayhierarchy.cpp:250-265, core/primitive.h:296-297).  The ray hierarchy
  * then groups rays by 2-D image tiles; 0, 0 clears the layout. */
 int pbg_preprocess(pbg_scene* scene, int64_t width, int64_t height);
+/* Declares how many samples of a pixel lie side by side in the camera batches
+ * that follow (Preprocess's samplesPerPixel); 0: not known.  Changes no result:
+ * ray-bvh's automatic walk asks for it. */
+int pbg_samples_per_pixel(pbg_scene* scene, int32_t samples);
 
 /* Nearest hit of n rays, host buffers in and out (copies included).
  * Replaces the batch Intersect of naive.cpp:204-338,

@@ -125,6 +125,7 @@ def lib():
     L.pbg_stats.argtypes = [vp, C.POINTER(Counters)]
     L.pbg_profile.argtypes = [vp, C.c_int]
     L.pbg_preprocess.argtypes = [vp, C.c_int64, C.c_int64]
+    L.pbg_samples_per_pixel.argtypes = [vp, C.c_int32]
     _lib = L
     return L
 

@@ -102,6 +102,7 @@ class Aggregate:
             self.tile = (xres // nx * samplesPerPixel, yres // ny)
             L.check(L.lib().pbg_preprocess(self.handle, self.tile[0], self.tile[1]),
                     "pbg_preprocess")
+            L.check(L.lib().pbg_samples_per_pixel(self.handle, samplesPerPixel), "pbg_samples_per_pixel")
 
     @staticmethod
     def _rays_struct(rays: np.ndarray, valid: np.ndarray | None) -> L.Rays:

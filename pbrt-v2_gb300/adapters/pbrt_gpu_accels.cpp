@@ -203,6 +203,7 @@ void preprocess(GpuAccel* g, const Camera* camera, unsigned spp, int nx, int ny)
     const int64_t w = (int64_t)(camera->film->xResolution / nx) * spp;
     const int64_t h = camera->film->yResolution / ny;
     check(pbg_preprocess(g->scene, w, h), "pbg_preprocess");
+    check(pbg_samples_per_pixel(g->scene, (int32_t)spp), "pbg_samples_per_pixel");
 }
 
 void destroy(const void* self) {

@@ -1442,6 +1442,15 @@ int pbg_preprocess(pbg_scene* s, int64_t width, int64_t height) {
     return PBG_OK;
 }
 
+int pbg_samples_per_pixel(pbg_scene* s, int32_t samples) {
+    if (!s || samples < 0) {
+        set_last_error("pbg_samples_per_pixel: bad arguments");
+        return PBG_ERR_INVALID_ARGUMENT;
+    }
+    s->samples = samples;
+    return PBG_OK;
+}
+
 int pbg_profile(pbg_scene* s, int on) {
     if (!s) return PBG_ERR_INVALID_ARGUMENT;
     cudaSetDevice(s->device);

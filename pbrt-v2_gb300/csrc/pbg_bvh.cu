@@ -13,6 +13,7 @@
 // of the BVH's top cut; an any-hit ray whose guess holds an occluder stops
 // there.
 #include <algorithm>
+#include <cmath>
 
 #include "pbg_internal.h"
 #include "pbg_learn.h"
@@ -421,34 +422,53 @@ static int walk_counter(pbg_scene* s, const QueueRef& q, unsigned long long** ne
     return PBG_OK;
 }
 
+// Whether packets (walk 4) pay for n camera rays.  A packet walks for 32 rays in
+// the caller's order: the fewer pixels they cover and the smaller the tree, the
+// more they share, and the batch has to fill the chip with packets.  The line
+// lies at n = 2^20 (a + b x + c x^2), x = sqrt(triangles / 2^20), by the samples
+// of a pixel that lie side by side (1; 2 or 3, or not known; 4 and more), fitted
+// to where the two walks' times cross on a 20,000- and a 181,250-triangle terrain
+// and 1,024,000 triangles of spheres.  Against walk 6, in 2^20 rays, measured
+// (line): 1 sample 1.4 (1.5) / 2.7 (2.6) / 4.9 (5.0), 2 samples 1.0 (1.0) / 1.5
+// (1.5) / 3.3 (3.3), 4 samples 0.9 (0.9) / 1.0 (1.0) / 2.0 (2.0); against walk 2:
+// 0.3 (0.3) / 0.95 (0.8) / 1.9 (2.0), 0.15 (0.15) / 0.55 (0.45) / 1.05 (1.1), 0.1
+// (0.1) / 0.45 (0.35) / 0.85 (0.85).  Times, us, walk 2 / 4 / 6:
+//   20,000     1 sample  99,918 113 / 152 /  79, 1,049,321 242 / 211 / 196, 4,199,058 688 / 501 / 624
+//              4 samples 99,552 126 / 121 /  75, 1,049,024 230 / 179 / 186, 4,197,284 618 / 435 / 584
+//   181,250    1 sample  99,918 170 / 289 / 116, 1,049,321 387 / 381 / 306, 4,199,058 1167 / 940 / 1013
+//              4 samples 99,552 158 / 215 / 105, 1,049,024 365 / 294 / 293, 4,197,284 1067 / 753 / 958
+//   1,024,000  1 sample  99,918 171 / 302 / 108, 1,049,321 534 / 608 / 421, 4,199,058 1680 / 1438 / 1346
+//              4 samples 99,552 169 / 259 / 110, 1,049,024 498 / 473 / 397, 4,197,284 1538 / 1124 / 1261
+// Over 132 such batches the walk chosen is at most 4 % off the better of its
+// two against walk 6, 7 % against walk 2.
+static bool packets_pay(const pbg_scene* s, int64_t n, bool wide) {
+    constexpr float kLine[2][3][3] = {{{0.f, 2.f, 0.f}, {0.f, 1.1f, 0.f}, {0.f, 0.85f, 0.f}},
+                                      {{0.9f, 4.2f, 0.f}, {0.9f, 0.8f, 1.6f}, {0.85f, 0.f, 1.15f}}};
+    const float* l = kLine[wide][s->samples == 1 ? 0 : s->samples < 4 ? 1 : 2];
+    const float x2 = (float)s->ntri * 0x1p-20f;
+    return (float)n >= 0x1p20f * (l[0] + l[1] * std::sqrt(x2) + l[2] * x2);
+}
+
 // The walk of a batch class (hint 1: incoherent) of n rays.
-constexpr int64_t kPacketRays = 3 << 18;   // camera rays that pay for packets
 constexpr int64_t kOwnTestRays = 1 << 18;  // shadow rays that pay for walk 5
 static int choose_walk(const pbg_scene* s, bool any, int hint, int64_t n) {
     if (s->params.walk != 0) return s->params.walk;
     const int tuned = s->tune.bvh_walk[any ? 1 : 0][hint == 1 ? 1 : 0];
     if (tuned != 0) return tuned;
     // Untuned.  Bounce rays and their shadows: 6.  Coherent batches: packets
-    // (camera) and the lanes' own tests (shadows) pay once the batch fills the
-    // chip several times over; below that a packet's one dependent walk is the
-    // whole time.  Measured on terrains of 20,000 and 181,250 triangles and
-    // 1,024,000 triangles of spheres, us:
-    //   camera 500 rays      walk 4 224 / 300 / 386, 6  39 /  61 /  62, 2  52 / 81 / 80
-    //   camera 480,000       walk 4 145 / 249 / 419, 6 108 / 164 / 216, 2 132 / 218 / 297
-    //   camera 1,048,576     walk 4 188 / 351 / 670, 6 186 / 308 / 472, 2 226 / 363 / 631
-    //   camera 4,194,304     walk 4 431 / 702 / 1272, 6 589 / 979 / 1541
-    //   shadow 500           walk 5  34 /  35 /  59, 6  31 /  35 /  62
-    //   shadow 50,000        walk 5  45 /  53 /  99, 6  41 /  50 /  97
-    //   shadow 480,000       walk 5  65 /  96 / 227, 6  73 / 104 / 233
-    //   shadow 4,194,304     walk 5 271 / 474 / 1481, 6 354 / 597 / 1714
-    // The camera line is for several samples a pixel, whose packets are denser
-    // than the ones above: the 1,228,800 rays of a frame of 640 x 480 x 4 take
-    // packets in 876 us a frame, walk 6 in 897.  A scene that
-    // has traced only small camera batches has no eight-wide tree yet: walk 2
-    // then, instead of building one.
+    // (camera, above) and the lanes' own tests (shadows) pay once the batch
+    // fills the chip; below that a packet's one dependent walk is the whole
+    // time.  Shadow rays on the scenes above, us:
+    //   500           walk 5  34 /  35 /  59, 6  31 /  35 /  62
+    //   50,000        walk 5  45 /  53 /  99, 6  41 /  50 /  97
+    //   480,000       walk 5  65 /  96 / 227, 6  73 / 104 / 233
+    //   4,194,304     walk 5 271 / 474 / 1481, 6 354 / 597 / 1714
+    // A scene that has traced only camera batches has no eight-wide tree yet:
+    // walk 2 below the packets' line then, instead of building one.
     if (hint == 1) return 6;
     if (any) return n < kOwnTestRays ? 6 : 5;
-    return n >= kPacketRays ? 4 : s->wide_state > 0 ? 6 : 2;
+    const bool wide = s->wide_state > 0;
+    return packets_pay(s, n, wide) ? 4 : wide ? 6 : 2;
 }
 
 // Walk 3 sorts the batch and the learned ordering records it, both for a

@@ -135,6 +135,7 @@ struct pbg_scene {
     struct pbg::Learner* learn = nullptr;
     struct pbg::RenderBuffers* render_bufs = nullptr;  // pbg_render's frame buffers, kept across frames
     int64_t image_w = 0, image_h = 0;  // ray-image layout from pbg_preprocess (0 = none)
+    int32_t samples = 0;               // of a pixel, side by side in camera batches (0 = not known)
     float scene_lo[3] = {0, 0, 0}, scene_hi[3] = {0, 0, 0};
     pbg::DeviceBuffer err;     // int[4] device status words
     int* mbox_host = nullptr;  // mapped pinned words the host reads status through

@@ -1145,8 +1145,13 @@ int render(pbg_scene* s, const pbg_camera* cam, const pbg_light* lights, int32_t
     // camera rays and their shadow rays are coherent, later bounces are not
     struct HintGuard {
         pbg_scene* s;
-        ~HintGuard() { s->walk_hint = -1; }
-    } hint_guard{s};
+        int32_t samples;
+        ~HintGuard() {
+            s->walk_hint = -1;
+            s->samples = samples;
+        }
+    } hint_guard{s, s->samples};
+    s->samples = stream ? 0 : rc.spp;
     cudaStream_t side = overlap ? B.side : st;
     bool pending[2] = {false, false};  // a resolve on the side stream still reads set k
     const uint32_t* nq_dev = nullptr;  // the queue's length on the device (nq: its upper bound)
