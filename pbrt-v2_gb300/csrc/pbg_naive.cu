@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(kNaiveThreads)
     WorkCount wc;
     Bundle bd;
     const bool bundle = make_bundle(active, o, d, nd, &bd);
+    const bool idle = __all_sync(full, done);  // no valid ray
 
     auto test = [&](const TriRec& tr) {
         if (STATS) wc.filt++;
@@ -373,13 +374,13 @@ __global__ void __launch_bounds__(kNaiveThreads)
     const int32_t u0 = (int32_t)((int64_t)unculled * blockIdx.y / gridDim.y);
     const int32_t u1 = (int32_t)((int64_t)unculled * (blockIdx.y + 1) / gridDim.y);
     for (int32_t j = u0; j < u1; j += kNaiveGroup) {
-        if (__all_sync(full, done)) break;
+        if (ANY ? __all_sync(full, done) : idle) break;
         load(j, min(kNaiveGroup, u1 - j));
         test_all(min(kNaiveGroup, u1 - j));
     }
     const int32_t g0 = min((int32_t)blockIdx.y * per_split, ngroups), g1 = min(g0 + per_split, ngroups);
     for (int32_t g = g0; g < g1; ++g) {
-        if (__all_sync(full, done)) break;
+        if (ANY ? __all_sync(full, done) : idle) break;
         const int32_t first = unculled + g * kNaiveGroup;
         const int32_t cnt = min(kNaiveGroup, ntri - first);
         unsigned meet = full, side = 0;  // lanes whose rays test every member; members that the others test too
