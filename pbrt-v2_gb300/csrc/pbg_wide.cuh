@@ -84,15 +84,16 @@ __global__ void __launch_bounds__(kWideThreads, kWideMinBlocks)
     const unsigned lt = (1u << lane) - 1u;
     __shared__ CoopWarp coop[COOP ? kWideThreads / 32 : 1];
     // eight hit bits in visiting order: bit k to bit k ^ order (a table: the
-    // three conditional swaps took 15 instructions a visit)
-    __shared__ uint8_t visit[8][256];
-    for (int i = threadIdx.x; i < 8 * 256; i += kWideThreads) {
-        uint32_t m = (uint32_t)i & 255u;
-        const uint32_t vo = (uint32_t)i >> 8;
-        if (vo & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
-        if (vo & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
-        if (vo & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
-        visit[vo][i & 255] = (uint8_t)m;
+    // three conditional swaps took 15 instructions a visit), made four entries
+    // to a word
+    __shared__ __align__(4) uint8_t visit[8][256];
+    for (int i = threadIdx.x; i < 8 * 64; i += kWideThreads) {
+        const uint32_t vo = (uint32_t)i >> 6;
+        uint32_t m = ((uint32_t)i & 63u) * 0x04040404u + 0x03020100u;
+        if (vo & 1u) m = ((m & 0x55555555u) << 1) | ((m >> 1) & 0x55555555u);
+        if (vo & 2u) m = ((m & 0x33333333u) << 2) | ((m >> 2) & 0x33333333u);
+        if (vo & 4u) m = ((m & 0x0f0f0f0fu) << 4) | ((m >> 4) & 0x0f0f0f0fu);
+        reinterpret_cast<uint32_t*>(visit)[i] = m;
     }
     __syncthreads();
     int2 stack[kWideStack];  // (child base, hits | imask << 8 | distance bits)
