@@ -86,8 +86,12 @@ __device__ __forceinline__ float beam_spread(float c, bool plain) {
 // for: its leaf build zeroes the traversal's words, its finalize kernel
 // publishes the status, its split tests take a leaf per warp while there are
 // few pairs, and its other kernels fewer CTAs; larger batches use memsets, a
-// kernel of its own and a pair per warp.  Frames of 131,400 / 256,000 / 700,000 rays: 452 / 618 /
-// 1,664 us in the first form, 469 / 624 / 1,439 in the second.
+// kernel of its own and a pair per warp.  A camera batch and two shadow batches
+// of 19,159 / 131,400 / 256,000 / 518,400 / 700,000 / 1,048,576 rays, us: on
+// 12,000 triangles 249 / 500 / 529 / 625 / 682 / 654 in the first form, 300 / 536
+// / 552 / 624 / 676 / 635 in the second, which meet at the line; on 181,250
+// triangles 483 / 785 / 853 / 1,024 / 1,078 / 1,121 and 475 / 780 / 840 / 995 /
+// 1,040 / 1,071.
 constexpr int64_t kFewRays = 1 << 19;
 // CTAs per SM of the level kernels where tune.rh_grid has none: 12 for small
 // batches (of 4, 12, 32: 175, 172, 177 us at 19,159 rays), 32 for others (best
@@ -520,7 +524,8 @@ __global__ void __launch_bounds__(256)
 // 2,430 us before, 1,680 now.  Pairs differ so much in work that dealing them
 // out by a fixed stride left a tail: any-hit 4 x 455 us, 386 from the counter.
 // Exact tests held back: 386 -> 321.  Leaf tests by (member, leaf) and
-// beam_misses: nearest 490 -> 440 and 656 -> 592.
+// beam_misses: nearest 490 -> 440 and 656 -> 592 (both in narrow leaves only for
+// nearest hits: kNarrow).
 constexpr int kSplitWarps = 8;
 constexpr int kSplitBlocks = 4;  // CTAs per SM, all resident: best of 4 (any-hit 1,283 us a frame), 5 (1,315), 6 (1,362)
 

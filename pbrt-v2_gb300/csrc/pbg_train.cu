@@ -16,8 +16,8 @@
 // about a microsecond each in one CTA per 128 records; the tensor pipe is
 // nearly idle.  The step it replaces ran each product, transpose, bias,
 // column sum and reduction as its own kernel (32 launches a step).  8 steps
-// of 8,192 records through pbg_learn_train, weights read back: 2,717 us
-// before, 232 us now (23 us a step on the device, 64 of 152 SMs).
+// of 8,192 records through pbg_learn_train, weights read back: 2,700 us
+// before, 228 us now (23 us a step on the device, 64 of 152 SMs).
 //
 // TMEM columns (512, one CTA per SM): [0, 256) the products in flight (layer
 // 1 at 0, layer 2 at 64, logits at 0 once both are read, dH2 at 0, dH1 at
